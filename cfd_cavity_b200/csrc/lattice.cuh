@@ -332,25 +332,75 @@ struct StepScalars {
 };
 
 // ---------------------------------------------------------------------------
+// Quotients by the lattice's constants cs^2 and cs^4, correctly rounded in two
+// operations: x / c = RN(x h + RN(x l)) with h = RN(1/c), l = RN(1/c - h) and
+// the outer sum one fused multiply-add (Brisebarre and Muller, "Correctly
+// Rounded Multiplication by Arbitrary Precision Constants", IEEE Trans.
+// Computers 57(2), 2008).  That holds for every x whose product x l is a
+// normal number: the binary64 constants are checked on all significands whose
+// quotient lies near a rounding boundary, the binary32 ones on every
+// significand (tests/test_const_div_cpu.py).  Below that range (|x| < 2^-968,
+// 2^-102 in binary32) the last bit may differ; the quotients are only added to
+// 1 or to a population, which absorb such a term.  The reference's expressions
+// divide about thirty times per node by these; a general division is some
+// twenty dependent operations and a branch, which cuts a node's code into
+// blocks that cannot overlap: with general divisions FP64 128 x 511 took 15.5 us
+// per step on a B200, with these 5.6 (16 x 40: 9.2 and 2.9; the block-refined
+// 64 x 256 in two levels 61 and 27 us per coarse step; 256 x 1024 in three,
+// FP32 / binary16, 91 and 75).
+// ---------------------------------------------------------------------------
+template <class A>
+struct CsInv;  // 1/cs^2 = I2H + I2L, 1/cs^4 = I4H + I4L
+template <>
+struct CsInv<double> {
+    static constexpr double I2H = 3.0, I2L = 0x1.8p-53, I4H = 9.0, I4L = 0x1.2p-51;
+};
+template <>
+struct CsInv<float> {
+    static constexpr float I2H = 3.0f, I2L = -0x1.8p-24f, I4H = 0x1.1ffffep+3f, I4L = 0x1.300004p-22f;
+};
+template <class A>
+__device__ __forceinline__ A mul_hl(A x, A h, A l) {
+    if constexpr (std::is_same<A, double>::value)
+        return __fma_rn(x, h, __dmul_rn(x, l));
+    else
+        return __fmaf_rn(x, h, __fmul_rn(x, l));
+}
+// x / cs^2, x / (2 cs^2), x / cs^4, x / (2 cs^4)
+#ifdef __CUDA_ARCH__
+#define CAV_OVER(NAME, S, H, L, C) \
+    template <class A>             \
+    __host__ __device__ __forceinline__ A NAME(A x) { return mul_hl<A>(x, A(S) * CsInv<A>::H, A(S) * CsInv<A>::L); }
+#else
+#define CAV_OVER(NAME, S, H, L, C) \
+    template <class A>             \
+    __host__ __device__ __forceinline__ A NAME(A x) { return x / (C); }
+#endif
+CAV_OVER(over_cs2, 1.0, I2H, I2L, A(CS2))
+CAV_OVER(over_2cs2, 0.5, I2H, I2L, A(2.0) * A(CS2))
+CAV_OVER(over_cs4, 1.0, I4H, I4L, A(CS2) * A(CS2))
+CAV_OVER(over_2cs4, 0.5, I4H, I4L, A(2.0) * A(CS2) * A(CS2))
+#undef CAV_OVER
+
+// ---------------------------------------------------------------------------
 // Equilibria.  In the unshifted (FP64) form the expressions are those of the
-// reference (feq form restated at src/uniform/tests.rs:314-316); the shifted
-// form returns feq_i - w_i from (drho = rho - 1, rho).
+// reference (feq form restated at src/uniform/tests.rs:314-316), its divisions
+// by cs^2 and cs^4 in the form above; the shifted form returns feq_i - w_i
+// from (drho = rho - 1, rho).
 // ---------------------------------------------------------------------------
 template <class A>
 __host__ __device__ __forceinline__ A feq_full(int i, A rho, A ux, A uy) {
-    const A cs2 = A(CS2);
     A eu = A(CX(i)) * ux + A(CY(i)) * uy;
     A u2 = ux * ux + uy * uy;
-    return A(WD(i)) * rho * (A(1.0) + eu / cs2 + eu * eu / (A(2.0) * cs2 * cs2) - u2 / (A(2.0) * cs2));
+    return A(WD(i)) * rho * (A(1.0) + over_cs2<A>(eu) + over_2cs4<A>(eu * eu) - over_2cs2<A>(u2));
 }
 
 template <class A>
 __host__ __device__ __forceinline__ A geq_full(int i, A t, A ux, A uy, int order) {
-    const A cs2 = A(CS2);
     A eu = A(CX(i)) * ux + A(CY(i)) * uy;
-    if (order == 1) return A(WD(i)) * t * (A(1.0) + eu / cs2);
+    if (order == 1) return A(WD(i)) * t * (A(1.0) + over_cs2<A>(eu));
     A u2 = ux * ux + uy * uy;
-    return A(WD(i)) * t * (A(1.0) + eu / cs2 + eu * eu / (A(2.0) * cs2 * cs2) - u2 / (A(2.0) * cs2));
+    return A(WD(i)) * t * (A(1.0) + over_cs2<A>(eu) + over_2cs4<A>(eu * eu) - over_2cs2<A>(u2));
 }
 
 // ---------------------------------------------------------------------------
@@ -699,7 +749,6 @@ __device__ __forceinline__ CollF<A> collide_f_pre(const A (&f)[Q], const Macro<A
     const A r = m.rho, u = m.ux, v = m.uy;
     if constexpr (!SHIFT) {
         // ---- FP64: expression order of the reference ----------------------
-        const double cs2 = CS2;
 #pragma unroll
         for (int i = 0; i < Q; ++i) o.d[i] = f[i] - feq_full<double>(i, r, u, v);
         const double* d_f = o.d;
@@ -709,15 +758,17 @@ __device__ __forceinline__ CollF<A> collide_f_pre(const A (&f)[Q], const Macro<A
         double pyy = ((((d_f[2] + d_f[3]) + d_f[4]) + d_f[6]) + d_f[7]) + d_f[8];
         double pi2 = pxx * pxx + 2.0 * pxy * pxy + pyy * pyy;
         double rho_m = r > 1e-12 ? r : 1e-12;
-        double s_mag = sqrt(pi2) / (2.0 * cs2 * c.tau_s * rho_m);
+        double s_mag = sqrt(pi2) / (2.0 * CS2 * c.tau_s * rho_m);
         double nut = nut_ovr ? double(*nut_ovr) : c.cs * c.cs * s_mag;
         o.nut = nut;
         double tau_plus = 0.5 + 3.0 * (c.nu + nut);
         double tau_minus = 0.5 + LAMBDA_TRT / (tau_plus - 0.5);
-        o.w1 = 0.5 * (1.0 / tau_plus + 1.0 / tau_minus);
-        o.w2 = 0.5 * (1.0 / tau_plus - 1.0 / tau_minus);
-        o.k1 = 1.0 - 0.5 / tau_minus;
-        o.k2 = 1.0 - 0.5 / tau_plus;
+        // (0.5 / tau is 0.5 times the rounded 1 / tau)
+        const double inv_p = 1.0 / tau_plus, inv_m = 1.0 / tau_minus;
+        o.w1 = 0.5 * (inv_p + inv_m);
+        o.w2 = 0.5 * (inv_p - inv_m);
+        o.k1 = 1.0 - 0.5 * inv_m;
+        o.k2 = 1.0 - 0.5 * inv_p;
     } else {
         o = collide_f_pre_lane<A>(f, m, c, nut_ovr);
     }
@@ -731,15 +782,14 @@ __device__ __forceinline__ A collide_f_post(A (&f)[Q], const CollF<A>& o, const 
                                             const StepScalars<A>& c, A temp) {
     const A r = m.rho, u = m.ux, v = m.uy;
     if constexpr (!SHIFT) {
-        const double cs2 = CS2;
         const double fyv = r * c.beta * 1.0 * (temp - 0.0);
         const double* d_f = o.d;
 #pragma unroll
         for (int i = 0; i < Q; ++i) {
             const double cx = CX(i), cy = CY(i);
             double ei_u = cx * u + cy * v;
-            double s_i = WD(i) * ((cy - v) / cs2 + ei_u * cy / (cs2 * cs2)) * fyv;
-            double s_minus = WD(i) * (cy / cs2) * fyv;
+            double s_i = WD(i) * (over_cs2<double>(cy - v) + over_cs4<double>(ei_u * cy)) * fyv;
+            double s_minus = WD(i) * (CY(i) / CS2) * fyv;
             double s_plus = s_i - s_minus;
             f[i] = f[i] + (-o.w1 * d_f[i] - o.w2 * d_f[OPP(i)] + o.k1 * s_minus + o.k2 * s_plus);
         }
@@ -810,9 +860,10 @@ __device__ __forceinline__ void collide_node_lane(L (&f)[Q], L (&g)[Q], const Ma
 
 // Wall-node equilibrium of g (apply_thermal_boundary_conditions,
 // src/uniform/solver.rs:957-970): geq(T_wall, 0, 0) = w_i T_wall.
+// (The bracket of geq_full is 1 at u = 0 in either order.)
 template <class A>
-__device__ __forceinline__ A geq_rest(int i, A t, int order) {
-    return geq_full<A>(i, t, A(0.0), A(0.0), order);
+__device__ __forceinline__ A geq_rest(int i, A t, int) {
+    return A(WD(i)) * t;
 }
 
 }  // namespace cav

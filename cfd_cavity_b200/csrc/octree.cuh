@@ -228,8 +228,8 @@ __device__ __forceinline__ void oct_collide(A (&f)[Q], A (&g)[Q], const Macro<A,
         for (int i = 0; i < Q; ++i) {
             const double cx = CX(i), cy = CY(i);
             const double ei_u = cx * u + cy * v;
-            const double s_i = WD(i) * ((cy - v) / CS2 + ei_u * cy / (CS2 * CS2)) * fyv;
-            const double s_minus = WD(i) * (cy / CS2) * fyv;
+            const double s_i = WD(i) * (over_cs2<double>(cy - v) + over_cs4<double>(ei_u * cy)) * fyv;
+            const double s_minus = WD(i) * (CY(i) / CS2) * fyv;
             const double s_plus = s_i - s_minus;
             fo[i] = f[i] + (-c.a_f * d_f[i] - c.b_f * d_f[OPP(i)] + c.c_m * s_minus + c.c_p * s_plus);
         }
@@ -470,7 +470,7 @@ __device__ __forceinline__ void bc_g(const LvlIO<St>& L, int x, int y, const Src
     }
     if (wall) {
 #pragma unroll
-        for (int i = 0; i < Q; ++i) g[i] = geq_full<A>(i, tw, A(0.0), A(0.0), 2);
+        for (int i = 0; i < Q; ++i) g[i] = geq_rest<A>(i, tw, 2);
     } else {
         const Src r = (xs == x && ys == y) ? own : src_of<COARSE>(L, xs, ys);
 #pragma unroll
