@@ -109,7 +109,6 @@ __global__ void __launch_bounds__(128) k_adj_step(const St* __restrict__ X, cons
                                                   const typename Fmt<St>::A* __restrict__ Xfy_pre) {
     using A = typename Fmt<St>::A;
     pdl_wait();
-    pdl_trigger();
     long long s;
     const StepScalars<A> c = table_scalars<A>(table, S, step_dev, j, &s);
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
@@ -198,7 +197,6 @@ __global__ void __launch_bounds__(256) k_fwd_slot(const St* __restrict__ src, St
                                                   int S, const long long* step_dev, long long j) {
     using A = typename Fmt<St>::A;
     pdl_wait();
-    pdl_trigger();
     long long s;
     const StepScalars<A> c = table_scalars<A>(table, S, step_dev, j, &s);
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;

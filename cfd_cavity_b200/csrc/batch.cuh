@@ -79,7 +79,6 @@ __global__ void __maxnreg__(56)
                const long long* __restrict__ step_dev) {
     using A = typename Fmt<St>::A;
     pdl_wait();
-    pdl_trigger();
     const long long s = step_dev ? *step_dev + step : step;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const BatchItem item = items[blockIdx.x];
@@ -106,7 +105,6 @@ __global__ void __maxnreg__(96)
                 const StepScalars<float>* __restrict__ table, int n_cav, long long step,
                 const long long* __restrict__ step_dev) {
     pdl_wait();
-    pdl_trigger();
     const long long s = step_dev ? *step_dev + step : step;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const BatchItem item = items[blockIdx.x];
@@ -123,15 +121,14 @@ __global__ void __maxnreg__(96)
 }
 
 // The node-pair body of k_fused_x (xpair.cuh: two x-adjacent nodes per
-// thread, every plane one 32-bit word) with one CTA per (cavity, 64-column x
-// rows) item: warp w takes row ty0 + w.  16-bit formats only.
+// thread, every plane one 32-bit word or float2) with one CTA per (cavity,
+// 64-column x rows) item: warp w takes row ty0 + w.
 template <class St, bool WRITE_NUT>
 __global__ void __maxnreg__(XPAIR_MAXNREG)
     k_batch_x(const BatchCav<St>* __restrict__ cavs, const BatchItem* __restrict__ items,
               const StepScalars<float>* __restrict__ table, int n_cav, long long step,
               const long long* __restrict__ step_dev) {
     pdl_wait();
-    pdl_trigger();
     const long long s = step_dev ? *step_dev + step : step;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const BatchItem item = items[blockIdx.x];
@@ -158,12 +155,12 @@ __global__ void __maxnreg__(XPAIR_MAXNREG)
 //                   lanes (rows_per_item in {2, 4, 8}; FP32-arithmetic formats);
 //   5  k_batch_x    one CTA per 64-column x rows_per_item item (rows_per_item
 //                   in {1, 2, 4, 8}), two x-adjacent nodes per thread, every
-//                   plane one 32-bit word (16-bit formats);
+//                   plane one 32-bit word (FP32: one float2; not FP64);
 //   6  k_tile_x     the node-pair body on TMA-staged shared-memory tiles of
 //                   64 columns x rows_per_item rows (4 or 8), ctas_per_sm
 //                   persistent CTAs per SM (16-bit formats).
 // A kernel a format has no version of runs as kernel 3 (FP64: 4, 5 and 6;
-// FP32: 5 and 6).  Parameters a kernel does not use are ignored.
+// FP32: 6).  Parameters a kernel does not use are ignored.
 struct BatchTuning {
     int rows_per_item = 4;
     int ctas_per_sm = 8;
@@ -337,7 +334,8 @@ struct Batch final : BatchBase {
 
     // The kernel this format runs for a requested one (see BatchTuning).
     static int effective_kernel(int k) {
-        if ((k == 5 || k == 6) && !is_p16<St>::value) k = 3;
+        if (k == 5 && !has_pairs<St>::value) k = 3;
+        if (k == 6 && !is_p16<St>::value) k = 3;
         if (k == 4 && !Fmt<St>::SHIFT) k = 3;
         return k;
     }
@@ -459,7 +457,7 @@ struct Batch final : BatchBase {
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        if constexpr (is_p16<St>::value) {
+        if constexpr (has_pairs<St>::value) {
             if (k == 5) {
                 CK(cudaLaunchKernelEx(&cfg, k_batch_x<St, WN>, (const BatchCav<St>*)d_cavs, (const BatchItem*)d_items,
                                       (const StepScalars<float>*)d_table, int(cv.size()), step, sdev));

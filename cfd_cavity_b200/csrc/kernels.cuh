@@ -124,12 +124,19 @@ __device__ __forceinline__ void store_planes(St* __restrict__ dst, const Geom& G
 }
 
 // Programmatic dependent launch: a kernel launched with the programmatic
-// stream-serialisation attribute may start while its predecessor finishes;
+// stream-serialisation attribute may be set up while its predecessor finishes;
 // it must not touch global memory before pdl_wait() (which returns once the
 // predecessor grid has completed and its writes are visible; a no-op without
-// the attribute).  pdl_trigger() lets the successor launch early.
+// the attribute).  The kernels leave the trigger to their exit: triggering
+// right after the wait brings the successor's CTAs onto the SMs while the
+// current step runs, where they only hold slots (B200, 128 x 512 f16sr 2.35 us
+// per step with the early trigger, 2.24 without; FP32 2.38 and 2.27; the
+// adjoint's reverse step 5.05 and 4.55; the octree's coarse step 66 and 63).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Barrier of one f warp and one g warp (or the halves of a CTA).
+__device__ __forceinline__ void named_bar_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
 
 static __global__ void k_set_step(long long* p, long long v) { *p = v; }
 static __global__ void k_add_step(long long* p, long long d) { *p += d; }
@@ -202,8 +209,13 @@ __device__ __forceinline__ void pull_g(const St* __restrict__ src, const Geom& G
     for (int i = 0; i < Q; ++i) {
         // wall columns read their own node (a valid address) and discard it
         const int idx = (Q + i) * P + (wall_col ? kg : kg - CX(i) - CY(i) * W);
-        const A v = LANE ? Fmt<St>::lload(src[idx], Q + i) : Fmt<St>::load(src[idx], Q + i);
-        g[i] = wall_col ? geq_rest<A>(i, tw, c.geq_order) : v;
+        g[i] = LANE ? Fmt<St>::lload(src[idx], Q + i) : Fmt<St>::load(src[idx], Q + i);
+    }
+    // after all the loads: a select beside each load lets the compiler put
+    // the load under the wall-column branch, one round trip after another
+    if (wall_col) {
+#pragma unroll
+        for (int i = 0; i < Q; ++i) g[i] = geq_rest<A>(i, tw, c.geq_order);
     }
 }
 
@@ -424,14 +436,15 @@ __device__ __forceinline__ void fused_pair(const St* __restrict__ src, St* __res
 //              body force rho beta along +y (the reference's Poiseuille
 //              test of the TRT + Guo collision, src/uniform/tests.rs:246-376,
 //              turned by 90 degrees).
-template <class St, bool WRITE_NUT, bool ACC_NU, bool NO_COLLIDE, bool CHANNEL = false>
-__global__ void __launch_bounds__(256) k_fused(const St* __restrict__ src, St* __restrict__ dst,
-                                               typename Fmt<St>::A* __restrict__ fy,
-                                               typename Fmt<St>::A* __restrict__ nut, double* __restrict__ acc_hot,
-                                               double* __restrict__ acc_cold, Geom G,
-                                               StepScalars<typename Fmt<St>::A> c) {
+template <class St, bool WRITE_NUT, bool ACC_NU, bool NO_COLLIDE, bool CHANNEL = false, int THREADS = 256,
+          int MIN_CTAS = 1>
+__global__ void __launch_bounds__(THREADS, MIN_CTAS) k_fused(const St* __restrict__ src, St* __restrict__ dst,
+                                                             typename Fmt<St>::A* __restrict__ fy,
+                                                             typename Fmt<St>::A* __restrict__ nut,
+                                                             double* __restrict__ acc_hot,
+                                                             double* __restrict__ acc_cold, Geom G,
+                                                             StepScalars<typename Fmt<St>::A> c) {
     pdl_wait();
-    pdl_trigger();
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ix >= G.nx || iy >= G.ny) return;

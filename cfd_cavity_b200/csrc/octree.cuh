@@ -492,7 +492,6 @@ __global__ void __launch_bounds__(OT) k_oct_step(LvlPair<St> P, const OctScal<ty
                                                  int S, const long long* __restrict__ step_dev, int off, int lvl,
                                                  uint32_t seed, int phase, float inv_nx, int collide) {
     pdl_wait();
-    pdl_trigger();
     using A = typename Fmt<St>::A;
     constexpr bool SH = Fmt<St>::SHIFT;
     const LvlIO<St> L = P.b[blockIdx.y];
@@ -549,7 +548,6 @@ __global__ void __launch_bounds__(2 * OCT_FG) k_oct_step_fg(LvlPair<St> P, const
                                                            int lvl, uint32_t seed, int phase, float inv_nx) {
     static_assert(Fmt<St>::SHIFT, "the split step runs the shifted formats");
     pdl_wait();
-    pdl_trigger();
     __shared__ float xu[OCT_FG], xv[OCT_FG], xq[OCT_FG], xt[OCT_FG];
     const LvlIO<St> L = P.b[blockIdx.y];
     const bool g_half = threadIdx.x >= OCT_FG;
@@ -623,7 +621,6 @@ __global__ void __launch_bounds__(OT) k_oct_collide(LvlPair<St> P, const OctScal
                                                     int S, const long long* __restrict__ step_dev, int lvl,
                                                     uint32_t seed, int phase, DynPtr<typename Fmt<St>::A> D) {
     pdl_wait();
-    pdl_trigger();
     using A = typename Fmt<St>::A;
     constexpr bool SH = Fmt<St>::SHIFT;
     const LvlIO<St> L = P.b[blockIdx.y];
@@ -749,7 +746,6 @@ __global__ void __launch_bounds__(OT) k_oct_c2f(LvlPair<StC> C, LvlPair<StF> F,
                                                 const Xi<typename Fmt<StF>::A>* __restrict__ xi_dev,
                                                 const long long* __restrict__ step_dev, uint32_t seed, int phase) {
     pdl_wait();
-    pdl_trigger();
     using A = typename Fmt<StF>::A;
     constexpr bool SH = Fmt<StF>::SHIFT;
     static_assert(Fmt<StC>::SHIFT == SH, "levels share one convention");
@@ -806,7 +802,6 @@ __global__ void __launch_bounds__(OT) k_oct_f2c(LvlPair<StF> F, LvlPair<StC> C, 
                                                 const long long* __restrict__ step_dev, int off, int lvl_c,
                                                 uint32_t seed, int phase, int collide) {
     pdl_wait();
-    pdl_trigger();
     using A = typename Fmt<StF>::A;
     constexpr bool SH = Fmt<StF>::SHIFT;
     // F2C_NPW coincident nodes per warp, three lanes each (lanes 30, 31 idle)

@@ -161,23 +161,33 @@ struct Impl final : Solver {
     bool pc_form = false;    // false: REF form in pop[cur]; true: PC form in pop[cur]
     bool ref_cached = false; // PC form with a materialized REF copy in pop[cur ^ 1]
     cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
-    // Block height: 32 x 4 for FP32 storage, 32 x 2 otherwise.  Measured on a
-    // B200 with graph-replayed programmatic-launch steps (the next step's
-    // CTAs are placed while the current step's are still resident, so the
-    // balance over SMs depends on the CTA count): FP32 128x512 2.24 us / step
-    // with 32 x 4 against 3.06 with 32 x 2; f16sr 2.47 with 32 x 2 against
-    // 2.51 with 32 x 4.
+    // Block height of the one-node kernels: 32 x 4 for FP32 storage, 32 x 2
+    // otherwise (a B200 takes about 1 us to start 1000 CTAs, so FP32's short
+    // steps want few; FP64's 156 registers leave 32 x 4 a coarser fit: 64 x 256
+    // 2.59 us against 2.54).
     static constexpr int BYF = std::is_same<St, float>::value ? 4 : BY;
     dim3 blk{BX, BYF}, grd{};
     // the node-pair kernel: 32 x BYX threads cover 64 columns x BYX rows
-    static constexpr int BYX = 2;
+    static constexpr int BYX = X_ROWS;
     dim3 blkx{BX, BYX}, grdx{};
     // the 16-bit formats' default step kernel: pairs split over two warps
     // for cavities that cannot fill the GPU (a step is then one thread's
-    // latency chain; on a B200 128 x 512 f16sr 2.32 us against 2.42, 64 x 256
-    // 1.67 against 2.00), plain pairs above (512 x 2048: 16.3 against 23.8)
+    // latency chain; on a B200 128 x 512 f16sr 2.25 us against 2.35, 64 x 256
+    // 1.74 against 2.00), plain pairs above (256 x 768: 4.2 against 5.1)
     static constexpr long long SPLIT_MAX_NODES = 70000;
     int kern = is_p16<St>::value ? 1 : 0;
+    // FP32 (step kernel 0): one node per thread while one thread's chain is
+    // all there is (96 x 384 1.80 us per step against 1.96 for split pairs),
+    // pairs split over two warps once issue counts too (128 x 512: 2.19 against
+    // 2.40), plain pairs above (512 x 1024: 8.8 against 9.2 and 11.6).
+    static constexpr long long F32_NODE_MAX = 48000;
+    int f32_form = 1;
+    // FP64: k_fused at 128 registers (8 CTAs of 64 threads per SM, a few
+    // words spilled) once the grid is more than the one wave that its 156
+    // registers leave room for (6 per SM): 128 x 511, 1024 CTAs, 4.50 us per
+    // step against 5.22; below that the spills cost (64 x 256: 2.67 against 2.54).
+    static constexpr int F64_CTAS = 6, F64_PACKED_CTAS = 8;
+    bool f64_packed = false;
     // dynamic subgrid model
     double dyn_alpha = 0.5, dyn_min = -0.1, dyn_eta = 2.0;
     double* sgs_w = nullptr;       // S_NPLANES FP64 work planes
@@ -208,6 +218,11 @@ struct Impl final : Solver {
         grd = dim3((p.nx + BX - 1) / BX, (p.ny + BYF - 1) / BYF);
         grdx = dim3(((p.nx + 1) / 2 + BX - 1) / BX, (p.ny + BYX - 1) / BYX);
         if (is_p16<St>::value && (long long)p.nx * p.ny <= SPLIT_MAX_NODES) kern = 2;
+        const long long nodes = (long long)p.nx * p.ny;
+        f32_form = nodes <= F32_NODE_MAX ? 0 : (nodes <= SPLIT_MAX_NODES ? 2 : 1);
+        int n_sm = 0;
+        CK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, p.device));
+        f64_packed = (long long)grd.x * grd.y > (long long)F64_CTAS * n_sm;
         if (!stream) {
             CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
             own_stream = true;
@@ -403,24 +418,36 @@ struct Impl final : Solver {
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        if constexpr (is_p16<St>::value) {
-            if (kern == 1) {
+        if constexpr (has_pairs<St>::value) {
+            if (form() == 1) {
                 cfg.gridDim = grdx;
                 cfg.blockDim = blkx;
                 CK(cudaLaunchKernelEx(&cfg, k_fused_x<St, WN, ACC, false>, (const St*)pop[cur], pop[cur ^ 1], fy,
                                       nut, acc_hot, acc_cold, G, c));
                 return;
             }
-            if (kern == 2) {
-                cfg.gridDim = dim3(((p.nx + 1) / 2 + 31) / 32, (p.ny + 1) / 2);
-                cfg.blockDim = dim3(128);
+            if (form() == 2) {
+                cfg.gridDim = dim3(((p.nx + 1) / 2 + 31) / 32, (p.ny + XS_ROWS - 1) / XS_ROWS);
+                cfg.blockDim = dim3(64 * XS_ROWS);
                 CK(cudaLaunchKernelEx(&cfg, k_fused_xs<St, WN, ACC>, (const St*)pop[cur], pop[cur ^ 1], fy, nut,
                                       acc_hot, acc_cold, G, c));
                 return;
             }
         }
+        if constexpr (std::is_same<St, double>::value) {
+            if (f64_packed) {
+                CK(cudaLaunchKernelEx(&cfg, k_fused<St, WN, ACC, false, false, BX * BY, F64_PACKED_CTAS>, (const St*)pop[cur],
+                                      pop[cur ^ 1], fy, nut, acc_hot, acc_cold, G, c));
+                return;
+            }
+        }
         CK(cudaLaunchKernelEx(&cfg, k_fused<St, WN, ACC, false>, (const St*)pop[cur], pop[cur ^ 1], fy, nut,
                               acc_hot, acc_cold, G, c));
+    }
+    // The kernel that runs a step: set_step_kernel's choice for the 16-bit
+    // formats; FP32 takes the node-pair kernels by size, FP64 one node per thread.
+    int form() const {
+        return is_p16<St>::value ? kern : (std::is_same<St, float>::value ? f32_form : 0);
     }
 
     void set_step_kernel(int k) override {
@@ -694,8 +721,8 @@ struct Impl final : Solver {
                 ref_cached = false;
                 for (int64_t j = 0; j < step_arg; ++j) {
                     bool done = false;
-                    if constexpr (is_p16<St>::value) {
-                        if (kern >= 1) {
+                    if constexpr (has_pairs<St>::value) {
+                        if (form() >= 1) {
                             k_fused_x<St, false, false, true><<<grdx, blkx, 0, stream>>>(
                                 pop[cur], pop[cur ^ 1], fy, nut, acc_hot, acc_cold, G, scalars(time_step));
                             done = true;

@@ -194,7 +194,6 @@ __global__ void __launch_bounds__(TileShape<St, V>::THREADS)
     }
     __syncthreads();
     pdl_wait();
-    pdl_trigger();
     const long long s = step_dev ? *step_dev + step : step;
     auto issue = [&](int item, int st) {
         const TileItem I = items[item];

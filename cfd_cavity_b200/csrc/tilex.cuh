@@ -146,7 +146,6 @@ __global__ void __launch_bounds__(TileXShape<TY>::THREADS, TileXShape<TY>::MIN_C
     }
     __syncthreads();
     pdl_wait();
-    pdl_trigger();
     const long long s = step_dev ? *step_dev + step : step;
     const int per = (n_items + int(gridDim.x) - 1) / int(gridDim.x);
     const int it0 = min(n_items, int(blockIdx.x) * per), it1 = min(n_items, it0 + per);

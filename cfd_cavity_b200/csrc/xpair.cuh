@@ -1,10 +1,10 @@
-// xpair.cuh -- the fused step on two x-adjacent nodes per thread (16-bit
-// population storage).
+// xpair.cuh -- the fused step on two x-adjacent nodes per thread (16-bit and
+// FP32 population storage).
 //
 // A thread owns the nodes (ix, iy) and (ix + 1, iy), ix even.  In the SoA
 // planes (pitch a multiple of 32 elements) those two 16-bit values are one
 // aligned 32-bit word, node ix in the low half, so every plane is pulled and
-// stored as words:
+// stored as words (FP32: aligned float2, the straddling pairs as two floats):
 //  - directions with c_x = 0: one word load (the source pair is aligned);
 //  - c_x = +1 / -1: the two source values straddle two words; both words are
 //    loaded and one byte permute (prmt) assembles the pair, with the
@@ -32,10 +32,29 @@ namespace cav {
 template <class St>
 struct PairEnc;
 
+// The formats the node-pair kernels run.
+template <class St>
+struct has_pairs : std::integral_constant<bool, is_p16<St>::value || std::is_same<St, float>::value> {};
+
+template <>
+struct PairEnc<float> {
+    using W = float2;  // a plane's values of the pair
+    static constexpr bool SR = false;
+    __device__ static float2 dec(float2 w, int) { return w; }
+    __device__ static void put(float* __restrict__ dst, int P, int k, int q, float2 v, uint32_t) {
+        *reinterpret_cast<float2*>(dst + q * P + k) = v;
+    }
+};
+
 template <int KIND, bool SRND>
 struct PairEnc<P16<KIND, SRND>> {
     using F = Fmt<P16<KIND, SRND>>;
+    using W = uint32_t;
     static constexpr bool SR = SRND;
+    // plane q of the pair at node offset k (even) of planes of P elements
+    __device__ static void put(P16<KIND, SRND>* __restrict__ dst, int P, int k, int q, float2 v, uint32_t r) {
+        reinterpret_cast<uint32_t*>(dst)[q * (P >> 1) + (k >> 1)] = enc(v, q, r);
+    }
     // lane units (the formats' own power-of-two scales), as Fmt::lload
     __device__ static float2 dec(uint32_t w, int q) {
         if constexpr (KIND == K_BF16) {
@@ -135,6 +154,48 @@ __device__ __forceinline__ void pull_g_x(const St* __restrict__ src, const Geom&
     }
 }
 
+// The same pulls from FP32 planes.
+__device__ __forceinline__ void pull_f_x(const float* __restrict__ s, const Geom& G, int ix, int iy, float2 (&w)[Q]) {
+    const int P = int(G.plane), W = G.pitch;
+    const int k = iy * W + ix;
+    const bool ym = iy > 0, yp = iy < G.ny - 1;
+    const bool x0 = ix == 0, xe = ix + 1 >= G.nx, xl = ix + 2 >= G.nx;
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+        const int cx = CX(i), cy = CY(i);
+        const bool y_ok = cy > 0 ? ym : (cy < 0 ? yp : true);
+        const int own = OPP(i) * P + k;
+        const int srow = i * P + k - cy * W;
+        if (cx == 0) {
+            w[i] = *reinterpret_cast<const float2*>(s + (y_ok ? srow : own));
+        } else if (cx > 0) {
+            w[i].x = s[(y_ok && !x0) ? srow - 1 : own];
+            w[i].y = s[y_ok ? srow : own + 1];
+        } else {
+            w[i].x = s[(y_ok && !xe) ? srow + 1 : own];
+            w[i].y = s[(y_ok && !xl) ? srow + 2 : own + 1];
+        }
+    }
+}
+__device__ __forceinline__ void pull_g_x(const float* __restrict__ s, const Geom& G, int ix, int iy, float2 (&w)[Q]) {
+    const int P = int(G.plane), W = G.pitch;
+    const int gy = iy == 0 ? 1 : (iy == G.ny - 1 ? G.ny - 2 : iy);
+    const int k = gy * W + ix;
+    const bool x0 = ix == 0, xl = ix + 2 >= G.nx;
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+        const int cx = CX(i), cy = CY(i);
+        const int srow = (Q + i) * P + k - cy * W;
+        if (cx == 0) {
+            w[i] = *reinterpret_cast<const float2*>(s + srow);
+        } else if (cx > 0) {
+            w[i] = make_float2(s[x0 ? srow : srow - 1], s[srow]);
+        } else {
+            w[i] = make_float2(s[srow + 1], s[xl ? srow : srow + 2]);
+        }
+    }
+}
+
 // Everything of one node-pair step after the pull: the macroscopic update
 // with the Guo half force, no-slip, the collision of the next step and the
 // stores (what fused_core does for one node).  pull_f(wf) / pull_g(wg) fill
@@ -156,7 +217,7 @@ __device__ __forceinline__ void xpair_core(PF&& pull_f, PG&& pull_g, TAt&& t_at,
     const int k0 = iy * G.pitch + ix;
     // f first: rho, u and the f collision's coefficients need no g
     float2 f[Q];
-    uint32_t wg[Q], wf[Q];
+    typename E::W wg[Q], wf[Q];
     pull_f(wf);
 #pragma unroll
     for (int i = 0; i < Q; ++i) f[i] = E::dec(wf[i], i);
@@ -192,8 +253,7 @@ __device__ __forceinline__ void xpair_core(PF&& pull_f, PG&& pull_g, TAt&& t_at,
     }
     // g collided and stored first (its registers free), then the f update;
     // stores: one word per plane, the draws in plane order 0..17
-    uint32_t* __restrict__ d = reinterpret_cast<uint32_t*>(dst);
-    const int P2 = int(G.plane >> 1), k2 = k0 >> 1;
+    const int P = int(G.plane);
     if (!NO_COLLIDE) {
         float2 qv[5];
         const float2 m15u2 = m15u2_lane<float2>(m.ux, m.uy);
@@ -209,10 +269,10 @@ __device__ __forceinline__ void xpair_core(PF&& pull_f, PG&& pull_g, TAt&& t_at,
         NodeRng rng = rng_f;
         rng.skip<Q>();
 #pragma unroll
-        for (int q = 0; q < Q; ++q) d[(Q + q) * P2 + k2] = E::enc(g[q], Q + q, rng.next());
+        for (int q = 0; q < Q; ++q) E::put(dst, P, k0, Q + q, g[q], rng.next());
     } else {
 #pragma unroll
-        for (int q = 0; q < Q; ++q) d[(Q + q) * P2 + k2] = E::enc(g[q], Q + q, 0u);
+        for (int q = 0; q < Q; ++q) E::put(dst, P, k0, Q + q, g[q], 0u);
     }
     if (!NO_COLLIDE) {
         const CollF<float2> o = collide_f_parts_lane<float2, EF>(f, m, kc);
@@ -222,10 +282,10 @@ __device__ __forceinline__ void xpair_core(PF&& pull_f, PG&& pull_g, TAt&& t_at,
     }
     if constexpr (E::SR) {
 #pragma unroll
-        for (int q = 0; q < Q; ++q) d[q * P2 + k2] = E::enc(f[q], q, rng_f.next());
+        for (int q = 0; q < Q; ++q) E::put(dst, P, k0, q, f[q], rng_f.next());
     } else {
 #pragma unroll
-        for (int q = 0; q < Q; ++q) d[q * P2 + k2] = E::enc(f[q], q, 0u);
+        for (int q = 0; q < Q; ++q) E::put(dst, P, k0, q, f[q], 0u);
     }
 }
 
@@ -239,8 +299,7 @@ __device__ __forceinline__ void fused_xpair(const St* __restrict__ src, St* __re
     const int k0 = iy * G.pitch + ix;
     const int gy = iy == 0 ? 1 : (iy == G.ny - 1 ? G.ny - 2 : iy);
     xpair_core<St, WRITE_NUT, ACC_NU, NO_COLLIDE>(
-        [&](uint32_t(&w)[Q]) { pull_f_x<St>(src, G, ix, iy, w); },
-        [&](uint32_t(&w)[Q]) { pull_g_x<St>(src, G, ix, iy, w); },
+        [&](auto& w) { pull_f_x(src, G, ix, iy, w); }, [&](auto& w) { pull_g_x(src, G, ix, iy, w); },
         [&](int x) { return gather_t<St>(src, G, x, iy, c); }, dst, *reinterpret_cast<const float2*>(fy_in + k0),
         c.t_hot[gy], fy_out, nut, acc_hot, acc_cold, G, ix, iy, c);
 }
@@ -254,10 +313,6 @@ __device__ __forceinline__ void fused_xpair(const St* __restrict__ src, St* __re
 // where a step is one thread's latency.  The same expressions in the same
 // order per node: bit-identical to k_fused_x.  CTA: 32 pairs x 2 rows x 2
 // roles (warps 0-1: f of rows 0-1; warps 2-3: g).
-__device__ __forceinline__ void named_bar_sync(int id, int threads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
 // The f half of a split node-pair step: pull of f, macroscopic update,
 // relaxation coefficients, publish (u, v, nu_t), named barrier `bar_id`
 // (64 threads: this warp and its g warp), read T, the f update and its
@@ -270,14 +325,13 @@ __device__ __forceinline__ void xpair_f_half(PF&& pull_f, float2* xu, float2* xv
                                              const StepScalars<float>& c) {
     using E = PairEnc<St>;
     constexpr int EF = Fmt<St>::EF, EG = Fmt<St>::EG;
-    const int k0 = iy * G.pitch + ix, k2 = k0 >> 1;
-    const int P2 = int(G.plane >> 1);
-    uint32_t* __restrict__ d = reinterpret_cast<uint32_t*>(dst);
+    const int k0 = iy * G.pitch + ix;
+    const int P = int(G.plane);
     float2 f[Q];
     Macro<float2, true> m{};
     CollCoef<float2> kc{};
     if (act) {
-        uint32_t wf[Q];
+        typename E::W wf[Q];
         pull_f(wf);
 #pragma unroll
         for (int i = 0; i < Q; ++i) f[i] = E::dec(wf[i], i);
@@ -299,10 +353,10 @@ __device__ __forceinline__ void xpair_f_half(PF&& pull_f, float2* xu, float2* xv
         if constexpr (E::SR) {
             NodeRng rng = sr_pair_rng(c, G, ix, iy);
 #pragma unroll
-            for (int q = 0; q < Q; ++q) d[q * P2 + k2] = E::enc(f[q], q, rng.next());
+            for (int q = 0; q < Q; ++q) E::put(dst, P, k0, q, f[q], rng.next());
         } else {
 #pragma unroll
-            for (int q = 0; q < Q; ++q) d[q * P2 + k2] = E::enc(f[q], q, 0u);
+            for (int q = 0; q < Q; ++q) E::put(dst, P, k0, q, f[q], 0u);
         }
     }
 }
@@ -319,12 +373,11 @@ __device__ __forceinline__ void xpair_g_half(PG&& pull_g, TAt&& t_at, float2* xt
                                              const StepScalars<float>& c) {
     using E = PairEnc<St>;
     constexpr int EG = Fmt<St>::EG;
-    const int k2 = (iy * G.pitch + ix) >> 1;
-    const int P2 = int(G.plane >> 1);
-    uint32_t* __restrict__ d = reinterpret_cast<uint32_t*>(dst);
+    const int k0 = iy * G.pitch + ix;
+    const int P = int(G.plane);
     float2 g[Q], t{};
     if (act) {
-        uint32_t wg[Q];
+        typename E::W wg[Q];
         pull_g(wg);
         const bool h0 = ix == 0, c0 = ix == G.nx - 1, c1 = ix + 1 == G.nx - 1;
         const float2 tw = make_float2((h0 ? t_hot_row : c.t_cold) * p2(EG), c.t_cold * p2(EG));
@@ -356,50 +409,52 @@ __device__ __forceinline__ void xpair_g_half(PG&& pull_g, TAt&& t_at, float2* xt
             NodeRng rng = sr_pair_rng(c, G, ix, iy);
             rng.skip<Q>();
 #pragma unroll
-            for (int q = 0; q < Q; ++q) d[(Q + q) * P2 + k2] = E::enc(g[q], Q + q, rng.next());
+            for (int q = 0; q < Q; ++q) E::put(dst, P, k0, Q + q, g[q], rng.next());
         } else {
 #pragma unroll
-            for (int q = 0; q < Q; ++q) d[(Q + q) * P2 + k2] = E::enc(g[q], Q + q, 0u);
+            for (int q = 0; q < Q; ++q) E::put(dst, P, k0, Q + q, g[q], 0u);
         }
     }
 }
 
+constexpr int XS_ROWS = 2;
 template <class St, bool WRITE_NUT, bool ACC_NU>
-__global__ void __launch_bounds__(128) k_fused_xs(const St* __restrict__ src, St* __restrict__ dst,
+__global__ void __launch_bounds__(64 * XS_ROWS) k_fused_xs(const St* __restrict__ src, St* __restrict__ dst,
                                                   float* __restrict__ fy, float* __restrict__ nut,
                                                   double* __restrict__ acc_hot, double* __restrict__ acc_cold, Geom G,
                                                   StepScalars<float> c) {
-    __shared__ float2 sh_t[2][32], sh_u[2][32], sh_v[2][32], sh_nut[2][32];
+    __shared__ float2 sh_t[XS_ROWS][32], sh_u[XS_ROWS][32], sh_v[XS_ROWS][32], sh_nut[XS_ROWS][32];
     pdl_wait();
-    pdl_trigger();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int r = w & 1, role = w >> 1;
+    const int r = w % XS_ROWS, role = w / XS_ROWS;
     const int ix = 2 * (blockIdx.x * 32 + lane);
-    const int iy = blockIdx.y * 2 + r;
+    const int iy = blockIdx.y * XS_ROWS + r;
     const bool act = ix < G.nx && iy < G.ny;
     if (role == 0) {
         const float2 fy_prev = act ? *reinterpret_cast<const float2*>(fy + iy * G.pitch + ix) : make_float2(0.f, 0.f);
-        xpair_f_half<St, WRITE_NUT>([&](uint32_t(&wf)[Q]) { pull_f_x<St>(src, G, ix, iy, wf); }, &sh_u[r][lane],
+        xpair_f_half<St, WRITE_NUT>([&](auto& wf) { pull_f_x(src, G, ix, iy, wf); }, &sh_u[r][lane],
                                     &sh_v[r][lane], &sh_nut[r][lane], &sh_t[r][lane], 1 + r, act, dst, fy_prev, fy,
                                     nut, G, ix, iy, c);
     } else {
         const int gy = iy == 0 ? 1 : (iy == G.ny - 1 ? G.ny - 2 : iy);
         const float th = (act && ix == 0) ? c.t_hot[gy] : 0.0f;
-        xpair_g_half<St, ACC_NU>([&](uint32_t(&wg)[Q]) { pull_g_x<St>(src, G, ix, iy, wg); },
+        xpair_g_half<St, ACC_NU>([&](auto& wg) { pull_g_x(src, G, ix, iy, wg); },
                                  [&](int x) { return gather_t<St>(src, G, x, iy, c); }, &sh_t[r][lane], &sh_u[r][lane],
                                  &sh_v[r][lane], &sh_nut[r][lane], 1 + r, act, dst, th, acc_hot, acc_cold, G, ix,
                                  iy, c);
     }
 }
-// The single-cavity step on node pairs: 32 x BY threads cover 64 columns x
-// BY rows.
+
+// The single-cavity step on node pairs: a CTA covers 64 columns x X_ROWS rows.
+// X_CTAS resident CTAs hold the registers to 96 (20 warps per SM): at 98 one
+// CTA fewer fits and 512 x 2048 f16sr takes 16.3 us instead of 15.6.
+constexpr int X_ROWS = 2, X_CTAS = 10;
 template <class St, bool WRITE_NUT, bool ACC_NU, bool NO_COLLIDE>
-__global__ void __launch_bounds__(256) k_fused_x(const St* __restrict__ src, St* __restrict__ dst,
+__global__ void __launch_bounds__(32 * X_ROWS, X_CTAS) k_fused_x(const St* __restrict__ src, St* __restrict__ dst,
                                                  float* __restrict__ fy, float* __restrict__ nut,
                                                  double* __restrict__ acc_hot, double* __restrict__ acc_cold, Geom G,
                                                  StepScalars<float> c) {
     pdl_wait();
-    pdl_trigger();
     const int ix = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ix >= G.nx || iy >= G.ny) return;
