@@ -7,7 +7,8 @@
 // `rows`-row) tiles: grid = ctas_per_sm x #SMs CTAs of 128 threads that
 // stride over the list.  Tiles are ordered cavity-major, row-block-minor, so
 // the tiles in flight at one time are neighbours and the halo rows they
-// share are served by L2.  Per-cavity step scalars (ramps, seeds, wall
+// share are served by L2.  A call's steps run group of cavities by group
+// (setup_groups), so that a group's state stays in the L2 between its steps.  Per-cavity step scalars (ramps, seeds, wall
 // temperature pointers) come from a device table precomputed on the host with
 // the single-cavity code (Impl::scalars), row min(step, spin_up), and every
 // node runs the same fused_node() as k_fused: a cavity advanced in a batch
@@ -37,6 +38,14 @@ struct BatchItem {
 };
 
 constexpr int BATCH_THREADS = 128;
+// Largest state of the cavities stepped together (Batch::setup_groups).  The
+// 64-cavity sweep (2.29 M nodes: 340 MB in FP32, 175 MB in 16 bits) on a B200,
+// us per lattice step against the groups' size in MB:
+//   FP32  (k_batch_np)      340: 61.9   85: 52.5   68: 46.3   57: 46.0   42: 47.4
+//   f16sr (k_batch_x, r 2)  175: 48.6   87: 43.8   58: 40.0   44: 41.5   35: 42.6
+// Above ~70 MB a group's planes push each other out of the 126 MB L2; small
+// groups pay each launch's start and last wave over fewer nodes.
+constexpr size_t GROUP_BYTES = 75'000'000;
 
 template <class St, bool WRITE_NUT>
 __global__ void __launch_bounds__(BATCH_THREADS)
@@ -193,8 +202,15 @@ struct Batch final : BatchBase {
     StepScalars<A>* d_table = nullptr;
     long long* step_dev = nullptr;
     long long step_dev_val = -1;
-    int n_items = 0, grid = 0, n_sm = 0, table_rows = 0;
-    cudaGraphExec_t graph = nullptr;
+    int n_sm = 0, table_rows = 0;
+    // Cavities [c0, c1) that are stepped together, their items in the work
+    // list of the current kernel, and GRAPH_STEPS of their steps as a graph
+    // (see setup_groups).
+    struct Group {
+        int c0, c1, item0 = 0, n_items = 0;
+        cudaGraphExec_t graph = nullptr;
+    };
+    std::vector<Group> groups;
     bool cavs_dirty = true;
     // the tile kernel (tile.cuh)
     TileCav<St>* d_tcavs = nullptr;
@@ -203,15 +219,17 @@ struct Batch final : BatchBase {
     CUtensorMap* d_xmaps[2] = {nullptr, nullptr};
     CUtensorMap* d_fmaps[2] = {nullptr, nullptr};  // the Guo force field of every cavity
     TileItem* d_xitems[2] = {nullptr, nullptr};
-    int n_xitems[2] = {0, 0}, xgrid = 0;
+    std::vector<int> xitem0[2];                             // first tile of every cavity, then their number
+    int occ = 0;                                            // resident CTAs per SM of the tile kernel in use
     TileItem* d_titems[3] = {nullptr, nullptr, nullptr};
     unsigned* d_err = nullptr;
     unsigned* h_err = nullptr;  // pinned copy of *d_err
-    int n_titems[3] = {0, 0, 0}, tgrid = 0;
+    std::vector<int> titem0[3];
     bool stall_copies = false;  // test of the bounded waits: arm the barriers, issue no copy
 
     ~Batch() override {
-        if (graph) cudaGraphExecDestroy(graph);
+        for (Group& g : groups)
+            if (g.graph) cudaGraphExecDestroy(g.graph);
         if (h_err) cudaFreeHost(h_err);
         void* bufs[] = {d_cavs,      d_items,     d_table, step_dev, d_tcavs,   d_maps[1],
                         d_maps[2],   d_titems[1], d_titems[2], d_err,  d_xmaps[0],
@@ -248,6 +266,7 @@ struct Batch final : BatchBase {
         CK(cudaMemsetAsync(d_err, 0, sizeof(unsigned), stream));
         CK(cudaMallocHost(&h_err, sizeof(unsigned)));
         *h_err = 0;
+        setup_groups();
         setup_tiles<1>();
         setup_tiles<2>();
         if constexpr (is_p16<St>::value) {
@@ -256,6 +275,35 @@ struct Batch final : BatchBase {
         }
         set_tuning(tun);
         CK(cudaStreamSynchronize(stream));
+    }
+
+    // The cavities are independent, so a call's steps are run for one group of
+    // them after another, each group small enough that its state stays in the
+    // L2 from step to step (126 MB; the rest is left to what else passes
+    // through), and about equal in size.
+    void setup_groups() {
+        auto bytes = [&](const Impl<St>* c) { return c->field_elems() * (2 * NPLANES * sizeof(St) + sizeof(A)); };
+        size_t total = 0;
+        for (auto* c : cv) total += bytes(c);
+        const size_t n = (total + GROUP_BYTES - 1) / GROUP_BYTES;
+        size_t done = 0, last = 0;
+        for (int i = 0; i < int(cv.size()); ++i) {
+            // a cavity goes with the group that its middle lies in
+            const size_t g = std::min(n - 1, (done + bytes(cv[i]) / 2) * n / total);
+            if (groups.empty() || g != last) groups.push_back(Group{i, i});
+            last = g;
+            groups.back().c1 = i + 1;
+            done += bytes(cv[i]);
+        }
+    }
+
+    // First item of every cavity (and the number of items) in a cavity-major list.
+    template <class Item>
+    std::vector<int> first_items(const std::vector<Item>& items) const {
+        std::vector<int> f(cv.size() + 1, 0);
+        for (const Item& it : items) ++f[it.cav + 1];
+        for (size_t i = 0; i < cv.size(); ++i) f[i + 1] += f[i];
+        return f;
     }
 
     // Tensor maps of both population buffers of every cavity and the tile
@@ -273,7 +321,7 @@ struct Batch final : BatchBase {
         for (auto* c : cv) sizes.push_back({c->p.nx, c->p.ny});
         std::vector<TileItem> ti;
         tile_items(sizes, TileShape<St, V>::TY, ti);
-        n_titems[V] = int(ti.size());
+        titem0[V] = first_items(ti);
         CK(cudaMalloc(&d_titems[V], sizeof(TileItem) * ti.size()));
         CK(cudaMemcpyAsync(d_titems[V], ti.data(), sizeof(TileItem) * ti.size(), cudaMemcpyHostToDevice, stream));
         CK(cudaFuncSetAttribute(k_tile<St, V, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -305,7 +353,7 @@ struct Batch final : BatchBase {
         for (auto* c : cv) sizes.push_back({c->p.nx, c->p.ny});
         std::vector<TileItem> ti;
         tilex_items(sizes, TY, ti);
-        n_xitems[slot] = int(ti.size());
+        xitem0[slot] = first_items(ti);
         CK(cudaMalloc(&d_xitems[slot], sizeof(TileItem) * ti.size()));
         CK(cudaMemcpyAsync(d_xitems[slot], ti.data(), sizeof(TileItem) * ti.size(), cudaMemcpyHostToDevice, stream));
         if constexpr (is_p16<St>::value) {
@@ -316,21 +364,24 @@ struct Batch final : BatchBase {
     }
 
     template <int TY>
-    int xtile_grid(int slot, int ctas_per_sm) {
-        int occ = 0;
+    int xtile_occ() {
+        int n = 1;
         if constexpr (is_p16<St>::value)
-            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tile_x<St, TY, false>, TileXShape<TY>::THREADS,
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_tile_x<St, TY, false>, TileXShape<TY>::THREADS,
                                                              TileXShape<TY>::SMEM));
-        return std::max(1, std::min(n_xitems[slot], std::max(1, std::min(ctas_per_sm, occ)) * n_sm));
+        return n;
     }
 
     template <int V>
-    int tile_grid(int ctas_per_sm) {
-        int occ = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_tile<St, V, false, false>, TileShape<St, V>::THREADS,
+    int tile_occ() {
+        int n = 1;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_tile<St, V, false, false>, TileShape<St, V>::THREADS,
                                                          TileShape<St, V>::SMEM));
-        return std::max(1, std::min(n_titems[V], std::max(1, std::min(ctas_per_sm, occ)) * n_sm));
+        return n;
     }
+
+    // Persistent CTAs over n work items.
+    int grid_of(int n) const { return std::max(1, std::min(n, std::max(1, std::min(tun.ctas_per_sm, occ)) * n_sm)); }
 
     // The kernel this format runs for a requested one (see BatchTuning).
     static int effective_kernel(int k) {
@@ -361,19 +412,34 @@ struct Batch final : BatchBase {
                 for (int x0 = 0; x0 < nx; x0 += width) items.push_back({i, x0, y0, std::min(r, ny - y0)});
         }
         if (d_items) CK(cudaFree(d_items));
-        n_items = int(items.size());
         CK(cudaMalloc(&d_items, sizeof(BatchItem) * items.size()));
         CK(cudaMemcpyAsync(d_items, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice,
                            stream));
-        grid = std::max(1, std::min(n_items, t.ctas_per_sm * n_sm));
-        if (t.kernel == 1) tgrid = tile_grid<1>(t.ctas_per_sm);
-        if (t.kernel == 2) tgrid = tile_grid<2>(t.ctas_per_sm);
-        if (k == 6) xgrid = r == 4 ? xtile_grid<4>(0, t.ctas_per_sm) : xtile_grid<8>(1, t.ctas_per_sm);
-        if (graph) {
-            cudaGraphExecDestroy(graph);
-            graph = nullptr;
+        occ = tun.ctas_per_sm;  // the persistent kernel 0: as asked
+        std::vector<int> first;
+        if (k == 1 || k == 2) {
+            first = titem0[k];
+            occ = k == 1 ? tile_occ<1>() : tile_occ<2>();
+        } else if (k == 6) {
+            first = xitem0[r == 4 ? 0 : 1];
+            occ = r == 4 ? xtile_occ<4>() : xtile_occ<8>();
+        } else {
+            first = first_items(items);
         }
+        for (Group& g : groups) {
+            g.item0 = first[g.c0];
+            g.n_items = first[g.c1] - first[g.c0];
+        }
+        drop_graphs();
         CK(cudaStreamSynchronize(stream));
+    }
+
+    void drop_graphs() {
+        for (Group& g : groups)
+            if (g.graph) {
+                cudaGraphExecDestroy(g.graph);
+                g.graph = nullptr;
+            }
     }
 
     // Brings every cavity to PC form at the shared step and refreshes the
@@ -427,9 +493,9 @@ struct Batch final : BatchBase {
     }
 
     template <int V, bool WN>
-    void launch_tiles(const long long* sdev, long long step) {
+    void launch_tiles(const Group& g, const long long* sdev, long long step) {
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(tgrid);
+        cfg.gridDim = dim3(grid_of(g.n_items));
         cfg.blockDim = dim3(TileShape<St, V>::THREADS);
         cfg.dynamicSmemBytes = TileShape<St, V>::SMEM;
         cfg.stream = stream;
@@ -439,16 +505,17 @@ struct Batch final : BatchBase {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         CK(cudaLaunchKernelEx(&cfg, k_tile<St, V, WN, false>, (const TileCav<St>*)d_tcavs,
-                              (const CUtensorMap*)d_maps[V], (const TileItem*)d_titems[V], n_titems[V],
+                              (const CUtensorMap*)d_maps[V], (const TileItem*)d_titems[V] + g.item0, g.n_items,
                               (const StepScalars<A>*)d_table, int(cv.size()), step, sdev, d_err,
                               int(stall_copies)));
     }
 
     // The one-CTA-per-item kernels (3, 4, 5) over d_items.
     template <bool WN>
-    void launch_np(int k, const long long* sdev, long long step) {
+    void launch_np(const Group& g, int k, const long long* sdev, long long step) {
+        const BatchItem* const items = d_items + g.item0;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(n_items);
+        cfg.gridDim = dim3(g.n_items);
         cfg.blockDim = dim3(32 * tun.rows_per_item);
         cfg.dynamicSmemBytes = 0;
         cfg.stream = stream;
@@ -459,7 +526,7 @@ struct Batch final : BatchBase {
         cfg.numAttrs = 1;
         if constexpr (has_pairs<St>::value) {
             if (k == 5) {
-                CK(cudaLaunchKernelEx(&cfg, k_batch_x<St, WN>, (const BatchCav<St>*)d_cavs, (const BatchItem*)d_items,
+                CK(cudaLaunchKernelEx(&cfg, k_batch_x<St, WN>, (const BatchCav<St>*)d_cavs, items,
                                       (const StepScalars<float>*)d_table, int(cv.size()), step, sdev));
                 return;
             }
@@ -468,20 +535,19 @@ struct Batch final : BatchBase {
             if (k == 4) {
                 cfg.blockDim = dim3(16 * tun.rows_per_item);
                 CK(cudaLaunchKernelEx(&cfg, k_batch_np2<St, WN>, (const BatchCav<St>*)d_cavs,
-                                      (const BatchItem*)d_items, (const StepScalars<float>*)d_table, int(cv.size()),
-                                      step, sdev));
+                                      items, (const StepScalars<float>*)d_table, int(cv.size()), step, sdev));
                 return;
             }
         }
-        CK(cudaLaunchKernelEx(&cfg, k_batch_np<St, WN>, (const BatchCav<St>*)d_cavs, (const BatchItem*)d_items,
+        CK(cudaLaunchKernelEx(&cfg, k_batch_np<St, WN>, (const BatchCav<St>*)d_cavs, items,
                               (const StepScalars<A>*)d_table, int(cv.size()), step, sdev));
     }
 
     template <int TY, bool WN>
-    void launch_xtiles(int slot, const long long* sdev, long long step) {
+    void launch_xtiles(const Group& g, int slot, const long long* sdev, long long step) {
         if constexpr (is_p16<St>::value) {
             cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(xgrid);
+            cfg.gridDim = dim3(grid_of(g.n_items));
             cfg.blockDim = dim3(TileXShape<TY>::THREADS);
             cfg.dynamicSmemBytes = TileXShape<TY>::SMEM;
             cfg.stream = stream;
@@ -492,59 +558,44 @@ struct Batch final : BatchBase {
             cfg.numAttrs = 1;
             CK(cudaLaunchKernelEx(&cfg, k_tile_x<St, TY, WN>, (const TileCav<St>*)d_tcavs,
                                   (const CUtensorMap*)d_xmaps[slot], (const CUtensorMap*)d_fmaps[slot],
-                                  (const TileItem*)d_xitems[slot], n_xitems[slot], (const StepScalars<float>*)d_table,
+                                  (const TileItem*)d_xitems[slot] + g.item0, g.n_items, (const StepScalars<float>*)d_table,
                                   int(cv.size()), step, sdev, d_err));
         }
     }
 
-    void launch(bool write_nut, const long long* sdev, long long step) {
+    template <bool WN>
+    void launch_kernel(const Group& g, const long long* sdev, long long step) {
         const int k = effective_kernel(tun.kernel);
         if (k == 6) {
-            if (tun.rows_per_item == 4)
-                write_nut ? launch_xtiles<4, true>(0, sdev, step) : launch_xtiles<4, false>(0, sdev, step);
-            else
-                write_nut ? launch_xtiles<8, true>(1, sdev, step) : launch_xtiles<8, false>(1, sdev, step);
-            ++launches;
-            CK(cudaGetLastError());
-            return;
+            tun.rows_per_item == 4 ? launch_xtiles<4, WN>(g, 0, sdev, step) : launch_xtiles<8, WN>(g, 1, sdev, step);
+        } else if (k >= 3) {
+            launch_np<WN>(g, k, sdev, step);
+        } else if (k >= 1) {
+            k == 1 ? launch_tiles<1, WN>(g, sdev, step) : launch_tiles<2, WN>(g, sdev, step);
+        } else {
+            k_batch<St, WN><<<grid_of(g.n_items), BATCH_THREADS, 0, stream>>>(
+                d_cavs, d_items + g.item0, g.n_items, d_table, int(cv.size()), step, sdev);
         }
-        if (k >= 3) {
-            write_nut ? launch_np<true>(k, sdev, step) : launch_np<false>(k, sdev, step);
-            ++launches;
-            CK(cudaGetLastError());
-            return;
-        }
-        if (tun.kernel == 1 || tun.kernel == 2) {
-            if (tun.kernel == 1)
-                write_nut ? launch_tiles<1, true>(sdev, step) : launch_tiles<1, false>(sdev, step);
-            else
-                write_nut ? launch_tiles<2, true>(sdev, step) : launch_tiles<2, false>(sdev, step);
-            ++launches;
-            CK(cudaGetLastError());
-            return;
-        }
-        if (write_nut)
-            k_batch<St, true><<<grid, BATCH_THREADS, 0, stream>>>(d_cavs, d_items, n_items, d_table, int(cv.size()),
-                                                                   step, sdev);
-        else
-            k_batch<St, false><<<grid, BATCH_THREADS, 0, stream>>>(d_cavs, d_items, n_items, d_table,
-                                                                    int(cv.size()), step, sdev);
+    }
+
+    void launch(const Group& g, bool write_nut, const long long* sdev, long long step) {
+        write_nut ? launch_kernel<true>(g, sdev, step) : launch_kernel<false>(g, sdev, step);
         ++launches;
         CK(cudaGetLastError());
     }
 
-    cudaGraphExec_t get_graph() {
-        if (graph) return graph;
+    cudaGraphExec_t get_graph(Group& g) {
+        if (g.graph) return g.graph;
         const int64_t l0 = launches;
         CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        for (int j = 0; j < GRAPH_STEPS; ++j) launch(false, step_dev, j);
+        for (int j = 0; j < GRAPH_STEPS; ++j) launch(g, false, step_dev, j);
         k_add_step<<<1, 1, 0, stream>>>(step_dev, GRAPH_STEPS);
         cudaGraph_t gr;
         CK(cudaStreamEndCapture(stream, &gr));
         launches = l0;
-        CK(cudaGraphInstantiate(&graph, gr, 0));
+        CK(cudaGraphInstantiate(&g.graph, gr, 0));
         cudaGraphDestroy(gr);
-        return graph;
+        return g.graph;
     }
 
     void advance_cavities(int64_t k) {
@@ -562,23 +613,30 @@ struct Batch final : BatchBase {
         for (auto* c : cv) entered_with_collide |= !c->pc_form;
         enter();  // may run one collision (the first step from a REF state)
         if (entered_with_collide) n -= 1;
+        if (n <= 0) return;
+        for (Group& g : groups) step_group(g, n);
+        advance_cavities(n);
+    }
+
+    // n steps of one group from the shared step (its cavities in PC form).
+    void step_group(Group& g, int64_t n) {
+        int64_t s = time_step;
+        if (n > GRAPH_STEPS && step_dev_val != s) {
+            k_set_step<<<1, 1, 0, stream>>>(step_dev, s);
+            CK(cudaGetLastError());
+            ++launches;
+            step_dev_val = s;
+        }
         while (n > 0) {
             if (n > GRAPH_STEPS) {
-                cudaGraphExec_t gx = get_graph();
-                if (step_dev_val != time_step) {
-                    k_set_step<<<1, 1, 0, stream>>>(step_dev, time_step);
-                    CK(cudaGetLastError());
-                    ++launches;
-                    step_dev_val = time_step;
-                }
-                CK(cudaGraphLaunch(gx, stream));
+                CK(cudaGraphLaunch(get_graph(g), stream));
                 launches += GRAPH_STEPS + 1;
                 step_dev_val += GRAPH_STEPS;
-                advance_cavities(GRAPH_STEPS);
+                s += GRAPH_STEPS;
                 n -= GRAPH_STEPS;
             } else {
-                launch(n == 1, nullptr, time_step);
-                advance_cavities(1);
+                launch(g, n == 1, nullptr, s);
+                s += 1;
                 n -= 1;
             }
         }
@@ -589,7 +647,8 @@ struct Batch final : BatchBase {
         cudaEvent_t a, b;
         CK(cudaEventCreate(&a));
         CK(cudaEventCreate(&b));
-        step(GRAPH_STEPS + 1);  // warm-up, builds the graph
+        // warm-up; the graphs only where the timed steps replay them
+        step(steps > GRAPH_STEPS ? GRAPH_STEPS + 1 : 4);
         CK(cudaEventRecord(a, stream));
         step(steps);
         CK(cudaEventRecord(b, stream));
@@ -618,10 +677,7 @@ struct Batch final : BatchBase {
     void set_stall_copies(bool on) override {
         CK(cudaStreamSynchronize(stream));
         stall_copies = on;
-        if (graph) {
-            CK(cudaGraphExecDestroy(graph));
-            graph = nullptr;
-        }
+        drop_graphs();
     }
 
     void sync() override { check_err(); }

@@ -118,8 +118,8 @@ __device__ __forceinline__ void pull_g_tx(const uint32_t* __restrict__ S, const 
 
 // One lattice step of every tile in `items` (x0 multiples of 64, y0 of TY;
 // cavity-major); step scalars of cavity c at step s are
-// table[min(s, spin_up) * n_cav + c].  CTA b takes the contiguous range of
-// tiles [b per, (b + 1) per), so consecutive tiles share the cavity (its
+// table[min(s, spin_up) * n_cav + c].  CTA b of B takes the contiguous range of
+// tiles [b n / B, (b + 1) n / B) (ranges differ by at most one tile), so consecutive tiles share the cavity (its
 // metadata is loaded once per range crossing) and their halo rows (L2).  Per
 // tile, the populations with their halo (maps[2 cav + buffer]) and the
 // previous Guo force of the tile (fmaps[cav]) arrive by TMA; the next tile's
@@ -147,8 +147,8 @@ __global__ void __launch_bounds__(TileXShape<TY>::THREADS, TileXShape<TY>::MIN_C
     __syncthreads();
     pdl_wait();
     const long long s = step_dev ? *step_dev + step : step;
-    const int per = (n_items + int(gridDim.x) - 1) / int(gridDim.x);
-    const int it0 = min(n_items, int(blockIdx.x) * per), it1 = min(n_items, it0 + per);
+    const int it0 = int((long long)n_items * blockIdx.x / gridDim.x);
+    const int it1 = int((long long)n_items * (blockIdx.x + 1) / gridDim.x);
     // the issuing thread's cavity and its buffer parity
     int icav = -1, ipar = 0;
     auto issue = [&](const TileItem& I, int st) {
