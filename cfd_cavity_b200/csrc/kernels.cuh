@@ -139,7 +139,10 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
 }
 
 static __global__ void k_set_step(long long* p, long long v) { *p = v; }
-static __global__ void k_add_step(long long* p, long long d) { *p += d; }
+static __global__ void k_add_step(long long* p, long long d) {
+    pdl_wait();
+    *p += d;
+}
 
 // Pull-stream of one node from a PC buffer (stream, solver.rs:838-913) fused
 // with the thermal boundary conditions (solver.rs:951-988):
@@ -455,21 +458,17 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) k_fused(const St* __restric
 // This is the reference's first phase of step() when the state comes from
 // new()/init_from_fields() or from the debug phases.
 template <class St>
-__global__ void __launch_bounds__(256) k_collide_ref(const St* __restrict__ src, St* __restrict__ dst,
-                                                     const typename Fmt<St>::A* __restrict__ rho,
-                                                     const typename Fmt<St>::A* __restrict__ ux,
-                                                     const typename Fmt<St>::A* __restrict__ uy,
-                                                     const typename Fmt<St>::A* __restrict__ tt,
-                                                     typename Fmt<St>::A* __restrict__ fy,
-                                                     typename Fmt<St>::A* __restrict__ nut, Geom G,
-                                                     StepScalars<typename Fmt<St>::A> c,
-                                                     const typename Fmt<St>::A* __restrict__ nut_pre = nullptr,
-                                                     const typename Fmt<St>::A* __restrict__ at_pre = nullptr) {
+__device__ __forceinline__ void collide_ref_node(const St* __restrict__ src, St* __restrict__ dst,
+                                                 const typename Fmt<St>::A* __restrict__ rho,
+                                                 const typename Fmt<St>::A* __restrict__ ux,
+                                                 const typename Fmt<St>::A* __restrict__ uy,
+                                                 const typename Fmt<St>::A* __restrict__ tt,
+                                                 typename Fmt<St>::A* __restrict__ fy,
+                                                 typename Fmt<St>::A* __restrict__ nut, const Geom& G, int ix, int iy,
+                                                 const StepScalars<typename Fmt<St>::A>& c,
+                                                 const typename Fmt<St>::A* nut_pre, const typename Fmt<St>::A* at_pre) {
     using A = typename Fmt<St>::A;
     constexpr bool SH = Fmt<St>::SHIFT;
-    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
-    const int iy = blockIdx.y * blockDim.y + threadIdx.y;
-    if (ix >= G.nx || iy >= G.ny) return;
     const long long k = (long long)iy * G.pitch + ix;
     A f[Q], g[Q];
 #pragma unroll
@@ -485,10 +484,31 @@ __global__ void __launch_bounds__(256) k_collide_ref(const St* __restrict__ src,
     m.uy = uy[k];
     m.t = tt[k];
     A fyv, nutv;
-    collide_node<A, SH>(f, g, m, c, fyv, nutv, nut_pre ? nut_pre + k : nullptr, at_pre ? at_pre + k : nullptr);
+    collide_node<A, SH>(f, g, m, c, fyv, nutv, nut_pre, at_pre);
     fy[k] = fyv;
     nut[k] = nutv;
     store_node<St>(dst, G, iy, ix, f, g, c);
+}
+
+// nut_pre, at_pre: nu_t and alpha_t per node (the dynamic model), or null.
+template <class St>
+__global__ void __launch_bounds__(256) k_collide_ref(const St* __restrict__ src, St* __restrict__ dst,
+                                                     const typename Fmt<St>::A* __restrict__ rho,
+                                                     const typename Fmt<St>::A* __restrict__ ux,
+                                                     const typename Fmt<St>::A* __restrict__ uy,
+                                                     const typename Fmt<St>::A* __restrict__ tt,
+                                                     typename Fmt<St>::A* __restrict__ fy,
+                                                     typename Fmt<St>::A* __restrict__ nut, Geom G,
+                                                     StepScalars<typename Fmt<St>::A> c,
+                                                     const typename Fmt<St>::A* __restrict__ nut_pre = nullptr,
+                                                     const typename Fmt<St>::A* __restrict__ at_pre = nullptr) {
+    pdl_wait();
+    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
+    const int iy = blockIdx.y * blockDim.y + threadIdx.y;
+    if (ix >= G.nx || iy >= G.ny) return;
+    const long long k = (long long)iy * G.pitch + ix;
+    collide_ref_node<St>(src, dst, rho, ux, uy, tt, fy, nut, G, ix, iy, c, nut_pre ? nut_pre + k : nullptr,
+                         at_pre ? at_pre + k : nullptr);
 }
 
 // PC(src) -> REF(dst): stream + thermal BC + macroscopic + no-slip, without
@@ -503,6 +523,7 @@ __global__ void __launch_bounds__(256) k_materialize(const St* __restrict__ src,
                                                      StepScalars<typename Fmt<St>::A> c) {
     using A = typename Fmt<St>::A;
     constexpr bool SH = Fmt<St>::SHIFT;
+    pdl_wait();
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ix >= G.nx || iy >= G.ny) return;
@@ -597,6 +618,7 @@ __global__ void k_acc_nu_pc(const St* __restrict__ src, double* __restrict__ acc
 template <class A>
 __global__ void k_acc_nu_ref(const A* __restrict__ tt, double* __restrict__ acc_hot, double* __restrict__ acc_cold,
                              Geom G) {
+    pdl_wait();
     const int iy = blockIdx.x * blockDim.x + threadIdx.x;
     if (iy >= G.ny) return;
     const long long r = (long long)iy * G.pitch;

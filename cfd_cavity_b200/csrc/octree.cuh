@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(OT) k_oct_step(LvlPair<St> P, const OctScal<ty
     pdl_wait();
     using A = typename Fmt<St>::A;
     constexpr bool SH = Fmt<St>::SHIFT;
-    const LvlIO<St> L = P.b[blockIdx.y];
+    const LvlIO<St> L = blockIdx.y == 0 ? P.b[0] : P.b[1];
     const int k = blockIdx.x * OT + threadIdx.x;
     if (k >= L.n) return;
     // the step index and the collision constants first: the stores below
@@ -549,7 +549,7 @@ __global__ void __launch_bounds__(2 * OCT_FG) k_oct_step_fg(LvlPair<St> P, const
     static_assert(Fmt<St>::SHIFT, "the split step runs the shifted formats");
     pdl_wait();
     __shared__ float xu[OCT_FG], xv[OCT_FG], xq[OCT_FG], xt[OCT_FG];
-    const LvlIO<St> L = P.b[blockIdx.y];
+    const LvlIO<St> L = blockIdx.y == 0 ? P.b[0] : P.b[1];
     const bool g_half = threadIdx.x >= OCT_FG;
     const int j = g_half ? threadIdx.x - OCT_FG : threadIdx.x;
     const int k = blockIdx.x * OCT_FG + j;
@@ -618,18 +618,18 @@ __global__ void __launch_bounds__(2 * OCT_FG) k_oct_step_fg(LvlPair<St> P, const
 // per-node nu_t / alpha_t of D).
 template <class St, bool COARSE>
 __global__ void __launch_bounds__(OT) k_oct_collide(LvlPair<St> P, const OctScal<typename Fmt<St>::A>* __restrict__ tab,
-                                                    int S, const long long* __restrict__ step_dev, int lvl,
-                                                    uint32_t seed, int phase, DynPtr<typename Fmt<St>::A> D) {
+                                                    int S, const long long* __restrict__ step_dev, int off,
+                                                    int lvl, uint32_t seed, int phase, DynPtr<typename Fmt<St>::A> D) {
     pdl_wait();
     using A = typename Fmt<St>::A;
     constexpr bool SH = Fmt<St>::SHIFT;
-    const LvlIO<St> L = P.b[blockIdx.y];
+    const LvlIO<St> L = blockIdx.y == 0 ? P.b[0] : P.b[1];
     const int k = blockIdx.x * OT + threadIdx.x;
     if (k >= L.n) return;
     const int x = k % L.nx, y = k / L.nx;
     if (!COARSE && (x == 0 || x == L.nx - 1 || y == 0 || y == L.ny - 1)) return;
     long long s;
-    const LvlScal<A> sc = row_of<A>(tab, S, step_dev, 0, &s).l[lvl];
+    const LvlScal<A> sc = row_of<A>(tab, S, step_dev, off, &s).l[lvl];
     A f[Q], g[Q];
     load_pops<St>(L.ref_in, L.n, k, f, g);
     Macro<A, SH> m;
@@ -640,8 +640,8 @@ __global__ void __launch_bounds__(OT) k_oct_collide(LvlPair<St> P, const OctScal
     m.uy = L.mac[2 * L.n + k];
     m.t = L.mac[3 * L.n + k];
     m.inv_rho = A(1.0) / m.rho;
-    const A* nut = D.nut[blockIdx.y];
-    const A* at = D.at[blockIdx.y];
+    const A* nut = blockIdx.y == 0 ? D.nut[0] : D.nut[1];
+    const A* at = blockIdx.y == 0 ? D.at[0] : D.at[1];
     A fy_new;
     oct_collide<A, SH>(f, g, m, sc, fy_new, nut ? nut + k : nullptr, at ? at + k : nullptr);
     L.fy[k] = fy_new;
@@ -744,7 +744,7 @@ __global__ void __launch_bounds__(OT) k_oct_c2f(LvlPair<StC> C, LvlPair<StF> F,
                                                 const GhostE<typename Fmt<StF>::A>* __restrict__ tab, int n_ghost,
                                                 Xi<typename Fmt<StF>::A> xi_h,
                                                 const Xi<typename Fmt<StF>::A>* __restrict__ xi_dev,
-                                                const long long* __restrict__ step_dev, uint32_t seed, int phase) {
+                                                const long long* __restrict__ step_dev, int off, uint32_t seed, int phase) {
     pdl_wait();
     using A = typename Fmt<StF>::A;
     constexpr bool SH = Fmt<StF>::SHIFT;
@@ -753,9 +753,9 @@ __global__ void __launch_bounds__(OT) k_oct_c2f(LvlPair<StC> C, LvlPair<StF> F,
     const int j = t >> 2, s = t & 3;
     if ((t & ~31) >= 4 * n_ghost) return;  // whole warp past the end
     const bool act = j < n_ghost;
-    const LvlIO<StC> Lc = C.b[blockIdx.y];
-    const LvlIO<StF> Lf = F.b[blockIdx.y];
-    const long long key = *step_dev * 16 + phase;
+    const LvlIO<StC> Lc = blockIdx.y == 0 ? C.b[0] : C.b[1];
+    const LvlIO<StF> Lf = blockIdx.y == 0 ? F.b[0] : F.b[1];
+    const long long key = (*step_dev + off) * 16 + phase;
     A c[NC];
     int kf = 0;
     if (act) {
@@ -812,8 +812,8 @@ __global__ void __launch_bounds__(OT) k_oct_f2c(LvlPair<StF> F, LvlPair<StC> C, 
     const int nb = blk == 0 ? n0 : n1;
     if (wi * F2C_NPW >= nb) return;  // whole warp past the end
     const bool act_e = lane < 3 * F2C_NPW && j < nb;
-    const LvlIO<StF> Lf = F.b[blk];
-    const LvlIO<StC> Lc = C.b[blk];
+    const LvlIO<StF> Lf = blk == 0 ? F.b[0] : F.b[1];
+    const LvlIO<StC> Lc = blk == 0 ? C.b[0] : C.b[1];
     CoinE e{0, 0, 0};
     if (act_e) e = tab[(blk == 0 ? 0 : n0) + j];
     long long sidx;
@@ -928,6 +928,7 @@ __device__ __forceinline__ double cta_max(double v, double* sh) {
 // part[(v * DYN_PARTS + b) * 2 + {0, 1}].
 template <class A>
 __global__ void __launch_bounds__(256) k_oct_mean_parts(XiJob<A> J, double* __restrict__ part) {
+    pdl_wait();
     __shared__ double sh[256];
     const MeanView<A> V = J.v[blockIdx.y];
     const int chunk = (V.n + DYN_PARTS - 1) / DYN_PARTS;
@@ -948,6 +949,7 @@ __global__ void __launch_bounds__(256) k_oct_mean_parts(XiJob<A> J, double* __re
 template <class A>
 __global__ void k_oct_xi(XiJob<A> J, const double* __restrict__ part, Xi<A>* __restrict__ xi_out,
                          double* __restrict__ xi_log) {
+    pdl_wait();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const int nv = J.mode == 0 ? 3 : 4;
     double mean[4][2];
@@ -999,6 +1001,7 @@ __global__ void k_oct_xi(XiJob<A> J, const double* __restrict__ part, Xi<A>* __r
 // order.
 static __global__ void __launch_bounds__(256) k_oct_sgs_parts(const double* __restrict__ W, int n,
                                                               double* __restrict__ part) {
+    pdl_wait();
     __shared__ double sh[256];
     const long long P = n;
     const int chunk = (n + DYN_PARTS - 1) / DYN_PARTS;
@@ -1764,9 +1767,13 @@ struct OctImpl final : Octree {
     // pdl_wait(), so a launch overlaps only the tail of its predecessor).
     template <typename... KArgs, typename... Args>
     void launch(void (*kern)(KArgs...), dim3 grid, Args... args) {
+        launch_b(kern, grid, dim3(OT), args...);
+    }
+    template <typename... KArgs, typename... Args>
+    void launch_b(void (*kern)(KArgs...), dim3 grid, dim3 block, Args... args) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = grid;
-        cfg.blockDim = dim3(OT);
+        cfg.blockDim = block;
         cfg.dynamicSmemBytes = 0;
         cfg.stream = stream;
         cudaLaunchAttribute attr[1];
@@ -1792,17 +1799,17 @@ struct OctImpl final : Octree {
         {
             LvlPair<StC> q = pair_cur(L0, L0);
             launch(k_oct_collide<StC, true>, grid_of(L0.n, 1), q, (const OctScal<A>*)tab, S,
-                   (const long long*)step_dev, 0, seed32, 10, DynPtr<A>{});
+                   (const long long*)step_dev, 0, 0, seed32, 10, DynPtr<A>{});
         }
         {
             LvlPair<StF> q = pair_cur(L1[0], L1[1]);
             launch(k_oct_collide<StF, false>, grid_of(L1[0].n, 2), q, (const OctScal<A>*)tab, S,
-                   (const long long*)step_dev, 1, seed32, 11, DynPtr<A>{});
+                   (const long long*)step_dev, 0, 1, seed32, 11, DynPtr<A>{});
         }
         if (levels == 3) {
             LvlPair<StF> q = pair_cur(L2[0], L2[1]);
             launch(k_oct_collide<StF, false>, grid_of(L2[0].n, 2), q, (const OctScal<A>*)tab, S,
-                   (const long long*)step_dev, 2, seed32, 12, DynPtr<A>{});
+                   (const long long*)step_dev, 0, 2, seed32, 12, DynPtr<A>{});
         }
         pc_valid = true;
     }
@@ -1814,17 +1821,18 @@ struct OctImpl final : Octree {
     const Xi<A>* xi_a_dev() const { return xi_dyn ? xi_dev : nullptr; }
     const Xi<A>* xi_b_dev() const { return xi_dyn ? xi_dev + 2 : nullptr; }
 
-    void c2f_L1() {
+    // j: coarse steps since *step_dev (replayed graphs hold several)
+    void c2f_L1(int j) {
         LvlPair<StC> c = pair_cur(L0, L0);
         LvlPair<StF> f = pair_cur(L1[0], L1[1]);
         launch(k_oct_c2f<StC, StF>, grid_of(4 * n_ghost, 2), c, f, (const GhostE<A>*)gh1, n_ghost, xa, xi_a_dev(),
-               (const long long*)step_dev, seed32, 2);
+               (const long long*)step_dev, j, seed32, 2);
     }
-    void c2f_L2() {
+    void c2f_L2(int j) {
         LvlPair<StF> c = pair_cur(L1[0], L1[1]);
         LvlPair<StF> f = pair_cur(L2[0], L2[1]);
         launch(k_oct_c2f<StF, StF>, grid_of(4 * n_ghost2, 2), c, f, (const GhostE<A>*)gh2, n_ghost2, xb, xi_b_dev(),
-               (const long long*)step_dev, seed32, 4);
+               (const long long*)step_dev, j, seed32, 4);
     }
     void f2c_L2(int off) {
         LvlPair<StF> f = pair_cur(L2[0], L2[1]);
@@ -1839,9 +1847,9 @@ struct OctImpl final : Octree {
         launch(k_oct_f2c<StF, StC>, f2c_grid(std::max(n_co0, n_co1)), f, c, (const CoinE*)co1, n_co0, n_co1,
                xa, xi_a_dev(), (const OctScal<A>*)tab, S, (const long long*)step_dev, off, 0, seed32, 13, int(!dyn));
     }
-    void step_L0() {
+    void step_L0(int j) {
         LvlPair<StC> q = pair(L0, L0);
-        launch(k_oct_step<StC, true>, grid_of(L0.n, 1), q, (const OctScal<A>*)tab, S, (const long long*)step_dev, 1,
+        launch(k_oct_step<StC, true>, grid_of(L0.n, 1), q, (const OctScal<A>*)tab, S, (const long long*)step_dev, j + 1,
                0, seed32, 1, 1.0f / float(L0.nx), int(!dyn));
         L0.cur ^= 1;
     }
@@ -1932,10 +1940,11 @@ struct OctImpl final : Octree {
         dyn_eta = eta_test;
     }
 
-    // The model on nb (1 or 2) blocks of one level shape in one launch per
-    // kernel (blockIdx.z = block).
-    template <class St>
-    void sgs_levels(const Lvl<St>* Ls, int nb, A* const* nuts, double tau_mol, double nu_l, double al_l) {
+    // The model on nb (1 or 2) blocks of one level shape (blockIdx.z = block)
+    // and the level's collision with its nu_t / alpha_t (REF -> PC).
+    template <bool COARSE, class St>
+    void sgs_levels(const Lvl<St>* Ls, int nb, A* const* nuts, double tau_mol, double nu_l, double al_l, int off,
+                    int lvl, int phase) {
         const Lvl<St>& L = Ls[0];
         const Geom G{L.nx, L.ny, L.nx, (long long)L.n};
         SgsParams sp;
@@ -1954,13 +1963,21 @@ struct OctImpl final : Octree {
             S.g[b] = SgsGrid<St>{Ls[b].ref[Ls[b].cur], mac,       mac + L.n, mac + 2 * L.n, mac + 3 * L.n,
                                  sgs_w + b * sgs_stride, nuts[b], nuts[b] + L.n};
         }
+        const LvlPair<St> q = pair_cur(Ls[0], Ls[nb - 1]);
         const dim3 blk(32, 4), grd((L.nx + 31) / 32, (L.ny + 3) / 4, nb);
-        k_sgs_b<St><<<grd, blk, 0, stream>>>(S, G, sp);
-        check_launch();
-        k_sgs_c<St><<<grd, blk, 0, stream>>>(S, G, sp);
-        check_launch();
-        k_sgs_d<St><<<grd, blk, 0, stream>>>(S, G, sp);
-        check_launch();
+        const bool w2 = sp.width == 2, half = sp.alpha_exp == 0.5;
+        launch_b(w2 ? k_sgs_b<St, 2> : k_sgs_b<St, 0>, grd, blk, S, G, sp);
+        launch_b(w2 ? (half ? k_sgs_c<St, 2, true> : k_sgs_c<St, 2, false>)
+                    : (half ? k_sgs_c<St, 0, true> : k_sgs_c<St, 0, false>),
+                 grd, blk, S, G, sp);
+        launch_b(w2 ? k_sgs_d<St, 2> : k_sgs_d<St, 0>, grd, blk, S, G, sp);
+        DynPtr<A> d{};
+        for (int b = 0; b < 2; ++b) {
+            d.nut[b] = S.g[std::min(b, nb - 1)].nut;
+            d.at[b] = S.g[std::min(b, nb - 1)].at;
+        }
+        launch(k_oct_collide<St, COARSE>, grid_of(L.n, nb), q, (const OctScal<A>*)tab, this->S,
+               (const long long*)step_dev, off, lvl, seed32, phase, d);
     }
 
     template <class St>
@@ -1983,14 +2000,13 @@ struct OctImpl final : Octree {
     // nu_t / alpha_t (REF -> PC), then pull + BC + macroscopic + no-slip
     // without the fused next collision; xi A / xi B from the mean effective
     // taus.  Host-driven launches (the model's constants follow the ramp).
-    void dyn_coarse_step() {
+    void dyn_coarse_step(int j) {
         xi_dyn = true;
         double nu_eff, al_eff;
-        ramp_of(time_step, nu_eff, al_eff);
+        ramp_of(time_step + j, nu_eff, al_eff);
         // L0 model, its coefficient statistics, xi A (L1 nu_t of the previous step)
-        sgs_levels(&L0, 1, &nut0, 0.5 + 3.0 * nu_eff, nu_eff, al_eff);
-        k_oct_sgs_parts<<<DYN_PARTS, 256, 0, stream>>>(sgs_w, L0.n, spart);
-        check_launch();
+        sgs_levels<true>(&L0, 1, &nut0, 0.5 + 3.0 * nu_eff, nu_eff, al_eff, j, 0, 1);
+        launch_b(k_oct_sgs_parts, dim3(DYN_PARTS), dim3(256), (const double*)sgs_w, L0.n, spart);
         {
             XiJob<A> J{};
             J.v[0] = mview(L0, nut0);
@@ -2002,22 +2018,14 @@ struct OctImpl final : Octree {
             J.nu_f = 2.0 * nu_eff;
             J.al_f = 2.0 * al_eff;
             J.odd_exact = p.odd_exact ? 1 : 0;
-            k_oct_mean_parts<A><<<dim3(DYN_PARTS, 3), 256, 0, stream>>>(J, mpart);
-            check_launch();
-            k_oct_xi<A><<<1, 32, 0, stream>>>(J, (const double*)mpart, xi_dev, dstat + 5);
-            check_launch();
+            launch_b(k_oct_mean_parts<A>, dim3(DYN_PARTS, 3), dim3(256), J, mpart);
+            launch_b(k_oct_xi<A>, dim3(1), dim3(32), J, (const double*)mpart, xi_dev, dstat + 5);
         }
-        const DynPtr<A> d0{{nut0, nut0}, {nut0 + L0.n, nut0 + L0.n}};
-        const DynPtr<A> d1{{nut1[0], nut1[1]}, {nut1[0] + L1[0].n, nut1[1] + L1[1].n}};
-        launch(k_oct_collide<StC, true>, grid_of(L0.n, 1), pair_cur(L0, L0), (const OctScal<A>*)tab, S,
-               (const long long*)step_dev, 0, seed32, 1, d0);
-        step_L0();
-        c2f_L1();
+        step_L0(j);
+        c2f_L1(j);
         const double tau_mol_l1 = 0.5 + 3.0 * 2.0 * nu_eff, tau_mol_l2 = 0.5 + 3.0 * 4.0 * nu_eff;
-        sgs_levels(L1, 2, nut1, tau_mol_l1, 2.0 * nu_eff, 2.0 * al_eff);
-        launch(k_oct_collide<StF, false>, grid_of(L1[0].n, 2), pair_cur(L1[0], L1[1]), (const OctScal<A>*)tab, S,
-               (const long long*)step_dev, 1, seed32, 3, d1);
-        step_L1(0, 3);
+        sgs_levels<false>(L1, 2, nut1, tau_mol_l1, 2.0 * nu_eff, 2.0 * al_eff, j, 1, 3);
+        step_L1(j, 3);
         if (levels == 3) {
             XiJob<A> J{};
             J.v[0] = mview(L1[0], nut1[0]);
@@ -2030,31 +2038,22 @@ struct OctImpl final : Octree {
             J.nu_f = 4.0 * nu_eff;
             J.al_f = 4.0 * al_eff;
             J.odd_exact = p.odd_exact ? 1 : 0;
-            k_oct_mean_parts<A><<<dim3(DYN_PARTS, 4), 256, 0, stream>>>(J, mpart);
-            check_launch();
-            k_oct_xi<A><<<1, 32, 0, stream>>>(J, (const double*)mpart, xi_dev + 2, dstat + 8);
-            check_launch();
-            c2f_L2();
-            const DynPtr<A> d2{{nut2[0], nut2[1]}, {nut2[0] + L2[0].n, nut2[1] + L2[1].n}};
+            launch_b(k_oct_mean_parts<A>, dim3(DYN_PARTS, 4), dim3(256), J, mpart);
+            launch_b(k_oct_xi<A>, dim3(1), dim3(32), J, (const double*)mpart, xi_dev + 2, dstat + 8);
+            c2f_L2(j);
             for (int sp = 0; sp < 2; ++sp) {
-                sgs_levels(L2, 2, nut2, tau_mol_l2, 4.0 * nu_eff, 4.0 * al_eff);
-                launch(k_oct_collide<StF, false>, grid_of(L2[0].n, 2), pair_cur(L2[0], L2[1]),
-                       (const OctScal<A>*)tab, S, (const long long*)step_dev, 2, seed32, 5 + sp, d2);
-                step_L2(0, 5 + sp);
+                sgs_levels<false>(L2, 2, nut2, tau_mol_l2, 4.0 * nu_eff, 4.0 * al_eff, j, 2, 5 + sp);
+                step_L2(j, 5 + sp);
             }
-            f2c_L2(0);
+            f2c_L2(j);
         }
         // the second L1 model takes the unramped nu / alpha (src/octree/solver.rs:882-890)
-        sgs_levels(L1, 2, nut1, tau_mol_l1, 2.0 * nu, 2.0 * alpha);
-        launch(k_oct_collide<StF, false>, grid_of(L1[0].n, 2), pair_cur(L1[0], L1[1]), (const OctScal<A>*)tab, S,
-               (const long long*)step_dev, 1, seed32, 9, d1);
-        step_L1(0, 9);
-        f2c_L1(0);
-        k_add_step<<<1, 1, 0, stream>>>(step_dev, 1);
-        check_launch();
+        sgs_levels<false>(L1, 2, nut1, tau_mol_l1, 2.0 * nu, 2.0 * alpha, j, 1, 9);
+        step_L1(j, 9);
+        f2c_L1(j);
     }
 
-    int64_t dyn_launches = 0;  // launches of one dynamic coarse step
+    int64_t dyn_launches = 0;  // launches of one dynamic graph
 
     void dynamic_stats(double* out) override {
         if (!dstat) {
@@ -2117,21 +2116,23 @@ struct OctImpl final : Octree {
     }
 
     // One step_cavity (src/octree/solver.rs:647-947), all launches on `stream`,
-    // with the step index taken from *step_dev (advanced at the end).
-    void launch_coarse_step() {
-        step_L0();
-        c2f_L1();
-        step_L1(0, 3);
+    // with the step index *step_dev + j.
+    void launch_coarse_step(int j) {
+        step_L0(j);
+        c2f_L1(j);
+        step_L1(j, 3);
         if (levels == 3) {
-            c2f_L2();
-            step_L2(0, 5);
-            step_L2(1, 6);
-            f2c_L2(0);
+            c2f_L2(j);
+            step_L2(j, 5);
+            step_L2(j + 1, 6);
+            f2c_L2(j);
         }
-        step_L1(1, 9);
-        f2c_L1(1);
-        k_add_step<<<1, 1, 0, stream>>>(step_dev, 1);
-        check_launch();
+        step_L1(j + 1, 9);
+        f2c_L1(j + 1);
+    }
+    // Advances *step_dev, once for all the steps launched since.
+    void add_steps(int n) {
+        launch_b(k_add_step, dim3(1), dim3(1), step_dev, (long long)n);
     }
 
     cudaGraphExec_t get_graph() {
@@ -2140,7 +2141,8 @@ struct OctImpl final : Octree {
         const int c0 = L0.cur, c1 = L1[0].cur, c2 = L2[0].cur;
         const int64_t l0 = launches;
         CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        for (int j = 0; j < OCT_GRAPH_STEPS; ++j) launch_coarse_step();
+        for (int j = 0; j < OCT_GRAPH_STEPS; ++j) launch_coarse_step(j);
+        add_steps(OCT_GRAPH_STEPS);
         cudaGraph_t gr;
         CK(cudaStreamEndCapture(stream, &gr));
         L0.cur = c0;
@@ -2152,7 +2154,7 @@ struct OctImpl final : Octree {
         return gx;
     }
 
-    int per_step_launches() const { return levels == 3 ? 10 : 6; }
+    int per_step_launches() const { return levels == 3 ? 9 : 5; }
 
     // OCT_GRAPH_STEPS dynamic coarse steps in one graph: valid once the
     // viscosity ramp has converged (the model's constants no longer change).
@@ -2162,10 +2164,13 @@ struct OctImpl final : Octree {
         const int c0 = L0.cur, c1 = L1[0].cur, c2 = L2[0].cur;
         const int64_t l0 = launches;
         CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        for (int j = 0; j < OCT_GRAPH_STEPS; ++j) dyn_coarse_step();
+        for (int j = 0; j < OCT_GRAPH_STEPS; ++j) {
+            dyn_coarse_step(0);
+            add_steps(1);
+        }
         cudaGraph_t gr;
         CK(cudaStreamEndCapture(stream, &gr));
-        dyn_launches = (launches - l0) / OCT_GRAPH_STEPS;
+        dyn_launches = launches - l0;
         L0.cur = c0;
         L1[0].cur = L1[1].cur = c1;
         L2[0].cur = L2[1].cur = c2;
@@ -2184,12 +2189,13 @@ struct OctImpl final : Octree {
                     const int64_t l0 = launches;
                     cudaGraphExec_t gx = get_dyn_graph();
                     CK(cudaGraphLaunch(gx, stream));
-                    launches = l0 + int64_t(OCT_GRAPH_STEPS) * dyn_launches;
+                    launches = l0 + dyn_launches;
                     xi_dyn = true;
                     time_step += OCT_GRAPH_STEPS;
                     n -= OCT_GRAPH_STEPS;
                 } else {
-                    dyn_coarse_step();
+                    dyn_coarse_step(0);
+                    add_steps(1);
                     time_step += 1;
                     n -= 1;
                 }
@@ -2204,11 +2210,12 @@ struct OctImpl final : Octree {
             if (n >= OCT_GRAPH_STEPS) {
                 cudaGraphExec_t gx = get_graph();
                 CK(cudaGraphLaunch(gx, stream));
-                launches += int64_t(OCT_GRAPH_STEPS) * per_step_launches();
+                launches += int64_t(OCT_GRAPH_STEPS) * per_step_launches() + 1;
                 time_step += OCT_GRAPH_STEPS;
                 n -= OCT_GRAPH_STEPS;
             } else {
-                launch_coarse_step();
+                launch_coarse_step(0);
+                add_steps(1);
                 time_step += 1;
                 n -= 1;
             }
@@ -2284,9 +2291,9 @@ struct OctImpl final : Octree {
     // 2 = coarse_to_fine L1 -> L2, 3 = fine_to_coarse L2 -> L1 (+ refresh).
     void debug_phase(int phase) override {
         set_step_dev();
-        if (phase == 0) c2f_L1();
+        if (phase == 0) c2f_L1(0);
         else if (phase == 1) f2c_L1(0);
-        else if (levels == 3 && phase == 2) c2f_L2();
+        else if (levels == 3 && phase == 2) c2f_L2(0);
         else if (levels == 3 && phase == 3) f2c_L2(0);
         else throw ArgError{CAV_ERR_ARG, "no such coupling phase"};
         pc_valid = false;

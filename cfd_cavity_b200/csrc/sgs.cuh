@@ -6,9 +6,9 @@
 // (compute_dynamic_sgs_level, src/octree/smag.rs:144-416: the same
 // algorithm with the level's tau, nu and alpha in its own lattice units).
 //
-// Three kernels, each one thread per node, every quantity in FP64 whatever
-// the storage format (the reference's arithmetic); a launch covers
-// gridDim.z grids of one shape (the two blocks of an octree level):
+// One thread per node, every quantity in FP64 whatever the storage format (the
+// reference's arithmetic); a launch covers gridDim.z grids of one shape (the two
+// blocks of an octree level).  Three kernels for any test-filter width:
 //   k_sgs_b  test-filter boxes of u_x, u_y, T (at the node and at the four
 //            neighbours its central differences read, each box summed in
 //            the reference's window order) and of the five products
@@ -22,9 +22,13 @@
 //   k_sgs_d  box of the numerators and denominators (regularisation),
 //            Lilly coefficients clamped to [0, 0.04], nu_t and alpha_t bounded
 //            below by the TRT floor, written for the collision.
+// The default width of two nodes (eta_test = 2) has its windows unrolled
+// (WIDTH 2).  The uniform solver then runs the first two parts as one kernel
+// (k_sgs_bc2) and the third inside the collision (k_sgs_collide2).
 // Sums run in the reference's order (box windows row by row), so every
-// quantity but the a^alpha powers (CUDA's pow, within 2 ulp of the
-// reference's) is bit-identical in FP64.
+// quantity but the a^alpha powers is bit-identical in FP64: CUDA's pow, within
+// 2 ulp of the reference's, or, at the default alpha = 1/2, one correctly
+// rounded square root of the product a b.
 #pragma once
 
 #include "kernels.cuh"
@@ -59,6 +63,8 @@ struct SgsGrid {
 template <class St>
 struct SgsGrids {
     SgsGrid<St> g[2];
+    // (selects: an indexed parameter would be copied to local memory)
+    __device__ __forceinline__ SgsGrid<St> at(int z) const { return z == 0 ? g[0] : g[1]; }
 };
 
 struct SgsParams {
@@ -127,170 +133,398 @@ __device__ __forceinline__ void box3(const A* __restrict__ ux, const A* __restri
     bt = s2 / w.cnt;
 }
 
+// What the first part of the model (k_sgs_b) gives for a node.
+struct SgsB {
+    double ubx, uby, tb, l[5];                                   // boxes of u_x, u_y, T and of the five products
+    double shxx, shxy, shyy, smh, sxx, sxy, syy, smb;            // grid- and test-level strain
+    double gtx, gty, gbx, gby, qsm, phi, tmh, tmb;
+};
+
+// Grid-level S~ and |S~| of a node from pi_neq, the collision's formula.
 template <class St>
-__global__ void __launch_bounds__(128) k_sgs_b(SgsGrids<St> S, Geom G, SgsParams sp) {
-    using A = typename Fmt<St>::A;
+__device__ __forceinline__ void sgs_strain(const SgsGrid<St>& io, const Geom& G, int ix, int iy, double ux_k,
+                                           double uy_k, const SgsParams& sp, SgsB& o) {
     constexpr bool SH = Fmt<St>::SHIFT;
-    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
-    const int iy = blockIdx.y * blockDim.y + threadIdx.y;
-    if (ix >= G.nx || iy >= G.ny) return;
-    const SgsGrid<St> io = S.g[blockIdx.z];
-    double* __restrict__ W = io.W;
+    const double rho_k = double(io.rho[iy * G.pitch + ix]) + sp.rho_off;
+    double pi_xx = 0.0, pi_xy = 0.0, pi_yy = 0.0;
+#pragma unroll
+    for (int i = 0; i < Q; ++i) {
+        const double fi = double(ldp(io.pops, G, i, iy, ix)) + (SH ? WD(i) : 0.0);
+        const double fneq = fi - feq_full<double>(i, rho_k, ux_k, uy_k);
+        if (CX(i) != 0) pi_xx += fneq;
+        if (CX(i) * CY(i) != 0) pi_xy += CX(i) * CY(i) > 0 ? fneq : -fneq;
+        if (CY(i) != 0) pi_yy += fneq;
+    }
+    const double rho_m = rho_k > 1e-12 ? rho_k : 1e-12;
+    const double denom = 2.0 * CS2 * sp.tau_s * rho_m;
+    const double pi2 = pi_xx * pi_xx + 2.0 * pi_xy * pi_xy + pi_yy * pi_yy;
+    o.shxx = -pi_xx / denom;
+    o.shxy = -pi_xy / denom;
+    o.shyy = -pi_yy / denom;
+    o.smh = sqrt(pi2) / denom;
+}
+
+// qsm^1/2 and Phi_sm^1/2 of a node from its fields and boxes.
+__device__ __forceinline__ void sgs_small(double u, double v, double t, double ub, double vb, double tb, double& q,
+                                          double& phi) {
+    const double du = u - ub, dv = v - vb;
+    const double r = sqrt(0.5 * (du * du + dv * dv));
+    q = r / 2.0;
+    phi = 0.5 * fabs(t - tb) * r;
+}
+
+// |T~| and |T-bar| from the gradients and strains.
+__device__ __forceinline__ void sgs_flux(SgsB& o) {
+    const double th_x = o.gtx * o.shxx + o.gty * o.shxy;
+    const double th_y = o.gtx * o.shxy + o.gty * o.shyy;
+    o.tmh = sqrt(2.0 * (th_x * th_x + th_y * th_y));
+    const double tb_x = o.gbx * o.sxx + o.gby * o.sxy;
+    const double tb_y = o.gbx * o.sxy + o.gby * o.syy;
+    o.tmb = sqrt(2.0 * (tb_x * tb_x + tb_y * tb_y));
+}
+
+// The first part for any test-filter width.
+template <class St>
+__device__ __forceinline__ void sgs_node_b(const SgsGrid<St>& io, const Geom& G, int ix, int iy, const SgsParams& sp,
+                                           SgsB& o) {
+    using A = typename Fmt<St>::A;
     const A* ux = io.ux;
     const A* uy = io.uy;
     const A* tt = io.tt;
-    const long long P = G.plane;
     const int k = iy * G.pitch + ix;
     // test-filter boxes at the node and at the neighbours of its central
     // differences (ddx / ddy clamp at the walls), and the Leonard boxes
     const int xm = ix == 0 ? 0 : ix - 1, xp = ix + 1 >= G.nx ? G.nx - 1 : ix + 1;
     const int ym = iy == 0 ? 0 : iy - 1, yp = iy + 1 >= G.ny ? G.ny - 1 : iy + 1;
-    double ubx, uby, tb, ubx_xm, uby_xm, tb_xm, ubx_xp, uby_xp, tb_xp, ubx_ym, uby_ym, tb_ym, ubx_yp, uby_yp, tb_yp;
-    box3<A>(ux, uy, tt, G, ix, iy, sp.width, ubx, uby, tb);
+    double ubx_xm, uby_xm, tb_xm, ubx_xp, uby_xp, tb_xp, ubx_ym, uby_ym, tb_ym, ubx_yp, uby_yp, tb_yp;
+    box3<A>(ux, uy, tt, G, ix, iy, sp.width, o.ubx, o.uby, o.tb);
     box3<A>(ux, uy, tt, G, xm, iy, sp.width, ubx_xm, uby_xm, tb_xm);
     box3<A>(ux, uy, tt, G, xp, iy, sp.width, ubx_xp, uby_xp, tb_xp);
     box3<A>(ux, uy, tt, G, ix, ym, sp.width, ubx_ym, uby_ym, tb_ym);
     box3<A>(ux, uy, tt, G, ix, yp, sp.width, ubx_yp, uby_yp, tb_yp);
-    {
-        const Window w = box_window(G, ix, iy, sp.width);
-        double l[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-        for (int yy = w.y0; yy < w.y1; ++yy)
-            for (int xx = w.x0; xx < w.x1; ++xx) {
-                const int kk = yy * G.pitch + xx;
-                const double u = ux[kk], v = uy[kk], t = tt[kk];
-                l[0] += u * u;
-                l[1] += u * v;
-                l[2] += v * v;
-                l[3] += u * t;
-                l[4] += v * t;
-            }
-        W[S_UBX * P + k] = ubx;
-        W[S_UBY * P + k] = uby;
-        W[S_TB * P + k] = tb;
-#pragma unroll
-        for (int p = 0; p < 5; ++p) W[(S_LXX + p) * P + k] = l[p] / w.cnt;
-    }
-    const double rho_k = double(io.rho[k]) + sp.rho_off, ux_k = ux[k], uy_k = uy[k], t_k = tt[k];
-    double pi_xx = 0.0, pi_xy = 0.0, pi_yy = 0.0;
-#pragma unroll
-    for (int i = 0; i < Q; ++i) {
-        const double cx = CX(i), cy = CY(i);
-        const double fi = double(ldp(io.pops, G, i, iy, ix)) + (SH ? WD(i) : 0.0);
-        const double fneq = fi - feq_full<double>(i, rho_k, ux_k, uy_k);
-        pi_xx += fneq * cx * cx;
-        pi_xy += fneq * cx * cy;
-        pi_yy += fneq * cy * cy;
-    }
-    const double rho_m = rho_k > 1e-12 ? rho_k : 1e-12;
-    const double denom = 2.0 * CS2 * sp.tau_s * rho_m;
-    const double pi2 = pi_xx * pi_xx + 2.0 * pi_xy * pi_xy + pi_yy * pi_yy;
-    const double shxx = -pi_xx / denom, shxy = -pi_xy / denom, shyy = -pi_yy / denom;
-    W[S_SHXX * P + k] = shxx;
-    W[S_SHXY * P + k] = shxy;
-    W[S_SHYY * P + k] = shyy;
-    W[S_SMH * P + k] = sqrt(pi2) / denom;
-    // ddx / ddy of the boxed fields (src/uniform/solver.rs:1229-1245)
-    const double sxx = 0.5 * (ubx_xp - ubx_xm);
-    const double syy = 0.5 * (uby_yp - uby_ym);
-    const double sxy = 0.5 * (0.5 * (uby_xp - uby_xm) + 0.5 * (ubx_yp - ubx_ym));
-    W[S_SBXX * P + k] = sxx;
-    W[S_SBXY * P + k] = sxy;
-    W[S_SBYY * P + k] = syy;
-    W[S_SMB * P + k] = sqrt(sxx * sxx + 2.0 * sxy * sxy + syy * syy);
-    const double gtx = ddx_f(tt, G, ix, iy), gty = ddy_f(tt, G, ix, iy);
-    const double gbx = 0.5 * (tb_xp - tb_xm), gby = 0.5 * (tb_yp - tb_ym);
-    W[S_GTX * P + k] = gtx;
-    W[S_GTY * P + k] = gty;
-    W[S_GBX * P + k] = gbx;
-    W[S_GBY * P + k] = gby;
-    const double dux = ux_k - ubx, duy = uy_k - uby;
-    const double du2 = dux * dux + duy * duy;
-    W[S_QSM * P + k] = sqrt(0.5 * du2) / 2.0;
-    const double dt_local = t_k - tb;
-    W[S_PHI * P + k] = 0.5 * fabs(dt_local) * sqrt(0.5 * du2);
-    const double th_x = gtx * shxx + gty * shxy;
-    const double th_y = gtx * shxy + gty * shyy;
-    W[S_TMH * P + k] = sqrt(2.0 * (th_x * th_x + th_y * th_y));
-    const double tb_x = gbx * sxx + gby * sxy;
-    const double tb_y = gbx * sxy + gby * syy;
-    W[S_TMB * P + k] = sqrt(2.0 * (tb_x * tb_x + tb_y * tb_y));
-}
-
-template <class St>
-__global__ void __launch_bounds__(128) k_sgs_c(SgsGrids<St> S, Geom G, SgsParams sp) {
-    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
-    const int iy = blockIdx.y * blockDim.y + threadIdx.y;
-    if (ix >= G.nx || iy >= G.ny) return;
-    double* __restrict__ W = S.g[blockIdx.z].W;
-    const long long P = G.plane;
-    const int k = iy * G.pitch + ix;
     const Window w = box_window(G, ix, iy, sp.width);
-    double sq = 0.0, sph = 0.0;
+    double l[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
     for (int yy = w.y0; yy < w.y1; ++yy)
         for (int xx = w.x0; xx < w.x1; ++xx) {
             const int kk = yy * G.pitch + xx;
-            sq += W[S_QSM * P + kk];
-            sph += W[S_PHI * P + kk];
+            const double u = ux[kk], v = uy[kk], t = tt[kk];
+            l[0] += u * u;
+            l[1] += u * v;
+            l[2] += v * v;
+            l[3] += u * t;
+            l[4] += v * t;
         }
-    const double qbar_h = sq / w.cnt, phibar_h = sph / w.cnt;
+#pragma unroll
+    for (int p = 0; p < 5; ++p) o.l[p] = l[p] / w.cnt;
+    const double ux_k = ux[k], uy_k = uy[k], t_k = tt[k];
+    sgs_strain<St>(io, G, ix, iy, ux_k, uy_k, sp, o);
+    // ddx / ddy of the boxed fields (src/uniform/solver.rs:1229-1245)
+    o.sxx = 0.5 * (ubx_xp - ubx_xm);
+    o.syy = 0.5 * (uby_yp - uby_ym);
+    o.sxy = 0.5 * (0.5 * (uby_xp - uby_xm) + 0.5 * (ubx_yp - ubx_ym));
+    o.smb = sqrt(o.sxx * o.sxx + 2.0 * o.sxy * o.sxy + o.syy * o.syy);
+    o.gtx = ddx_f(tt, G, ix, iy);
+    o.gty = ddy_f(tt, G, ix, iy);
+    o.gbx = 0.5 * (tb_xp - tb_xm);
+    o.gby = 0.5 * (tb_yp - tb_ym);
+    sgs_small(ux_k, uy_k, t_k, o.ubx, o.uby, o.tb, o.qsm, o.phi);
+    sgs_flux(o);
+}
+
+// The first part for the test filter of two nodes: the box of a node covers it
+// and its upper neighbours in x and y, cut at the grid's edge, its count (1, 2
+// or 4) divided out exactly by a multiplication.  The boxes a node needs -- its
+// own, those of the four neighbours that its central differences read (the
+// clamped ones are its own) and that of the diagonal one of its window -- all
+// come from 13 nodes, kept in registers.  WINDOW: also the boxes of qsm^1/2
+// and Phi_sm^1/2 at the node (from the four nodes of its window).
+template <class St, bool WINDOW>
+__device__ __forceinline__ void sgs_node_b2(const SgsGrid<St>& io, const Geom& G, int ix, int iy, const SgsParams& sp,
+                                            SgsB& o, double& qbar_h, double& phibar_h) {
+    const int k = iy * G.pitch + ix;
+    // offsets of columns ix - 1 .. ix + 2 and rows iy - 1 .. iy + 2, kept in
+    // the grid (values taken from a clamped place are not used)
+    const bool x0 = ix == 0, y0 = iy == 0;
+    const bool x1 = ix + 1 < G.nx, y1 = iy + 1 < G.ny, x2 = ix + 2 < G.nx, y2 = iy + 2 < G.ny;
+    const int ox[4] = {x0 ? 0 : -1, 0, x1 ? 1 : 0, x2 ? 2 : 0};
+    const int oy[4] = {y0 ? 0 : -G.pitch, 0, y1 ? G.pitch : 0, y2 ? 2 * G.pitch : 0};
+    // the box's mean of four values in window order; vx / vy: the second
+    // column / row is in the grid
+    auto box = [](double a, double b, double c, double d, bool vx, bool vy) {
+        const double s = ((a + (vx ? b : 0.0)) + (vy ? c : 0.0)) + (vx && vy ? d : 0.0);
+        return s * ((vx ? 0.5 : 1.0) * (vy ? 0.5 : 1.0));
+    };
+    struct Boxes {
+        double c, w, e, s, n, ne;
+    };
+    double uv[4][4], vv[4][4], tv[4][4];  // [row][column]; the corners no box reads stay unused
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if ((j == 0 && (i == 0 || i == 3)) || (j == 3 && i == 0)) continue;
+            const int kk = k + oy[j] + ox[i];
+            uv[j][i] = io.ux[kk];
+            vv[j][i] = io.uy[kk];
+            tv[j][i] = io.tt[kk];
+        }
+    auto boxes = [&](const double (&p)[4][4]) {
+        Boxes b;
+        b.c = box(p[1][1], p[1][2], p[2][1], p[2][2], x1, y1);
+        const double w = box(p[1][0], p[1][1], p[2][0], p[2][1], true, y1);
+        const double e = box(p[1][2], p[1][3], p[2][2], p[2][3], x2, y1);
+        const double s = box(p[0][1], p[0][2], p[1][1], p[1][2], x1, true);
+        const double n = box(p[2][1], p[2][2], p[3][1], p[3][2], x1, y2);
+        b.ne = box(p[2][2], p[2][3], p[3][2], p[3][3], x2, y2);
+        b.w = x0 ? b.c : w;
+        b.e = x1 ? e : b.c;
+        b.s = y0 ? b.c : s;
+        b.n = y1 ? n : b.c;
+        return b;
+    };
+    const Boxes bu = boxes(uv), bv = boxes(vv), bt = boxes(tv);
+    o.ubx = bu.c;
+    o.uby = bv.c;
+    o.tb = bt.c;
+    auto box_prod = [&](const double (&p)[4][4], const double (&q)[4][4]) {
+        return box(p[1][1] * q[1][1], p[1][2] * q[1][2], p[2][1] * q[2][1], p[2][2] * q[2][2], x1, y1);
+    };
+    o.l[0] = box_prod(uv, uv);
+    o.l[1] = box_prod(uv, vv);
+    o.l[2] = box_prod(vv, vv);
+    o.l[3] = box_prod(uv, tv);
+    o.l[4] = box_prod(vv, tv);
+    const double t_k = tv[1][1];
+    sgs_strain<St>(io, G, ix, iy, uv[1][1], vv[1][1], sp, o);
+    o.sxx = 0.5 * (bu.e - bu.w);
+    o.syy = 0.5 * (bv.n - bv.s);
+    o.sxy = 0.5 * (0.5 * (bv.e - bv.w) + 0.5 * (bu.n - bu.s));
+    o.smb = sqrt(o.sxx * o.sxx + 2.0 * o.sxy * o.sxy + o.syy * o.syy);
+    o.gtx = 0.5 * ((x1 ? tv[1][2] : t_k) - (x0 ? t_k : tv[1][0]));
+    o.gty = 0.5 * ((y1 ? tv[2][1] : t_k) - (y0 ? t_k : tv[0][1]));
+    o.gbx = 0.5 * (bt.e - bt.w);
+    o.gby = 0.5 * (bt.n - bt.s);
+    sgs_small(uv[1][1], vv[1][1], t_k, bu.c, bv.c, bt.c, o.qsm, o.phi);
+    if constexpr (WINDOW) {
+        double q1, q2, q3, p1, p2, p3;
+        sgs_small(uv[1][2], vv[1][2], tv[1][2], bu.e, bv.e, bt.e, q1, p1);
+        sgs_small(uv[2][1], vv[2][1], tv[2][1], bu.n, bv.n, bt.n, q2, p2);
+        sgs_small(uv[2][2], vv[2][2], tv[2][2], bu.ne, bv.ne, bt.ne, q3, p3);
+        qbar_h = box(o.qsm, q1, q2, q3, x1, y1);
+        phibar_h = box(o.phi, p1, p2, p3, x1, y1);
+    }
+    sgs_flux(o);
+}
+
+template <class St, int WIDTH>
+__global__ void __launch_bounds__(128) k_sgs_b(SgsGrids<St> S, Geom G, SgsParams sp) {
+    pdl_wait();
+    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
+    const int iy = blockIdx.y * blockDim.y + threadIdx.y;
+    if (ix >= G.nx || iy >= G.ny) return;
+    const SgsGrid<St> io = S.at(blockIdx.z);
+    SgsB o;
+    if constexpr (WIDTH == 2) {
+        double qb, pb;
+        sgs_node_b2<St, false>(io, G, ix, iy, sp, o, qb, pb);
+    } else {
+        sgs_node_b<St>(io, G, ix, iy, sp, o);
+    }
+    const long long P = G.plane;
+    double* __restrict__ w = io.W + iy * G.pitch + ix;
+    w[S_UBX * P] = o.ubx;
+    w[S_UBY * P] = o.uby;
+    w[S_TB * P] = o.tb;
+#pragma unroll
+    for (int p = 0; p < 5; ++p) w[(S_LXX + p) * P] = o.l[p];
+    w[S_SHXX * P] = o.shxx;
+    w[S_SHXY * P] = o.shxy;
+    w[S_SHYY * P] = o.shyy;
+    w[S_SMH * P] = o.smh;
+    w[S_SBXX * P] = o.sxx;
+    w[S_SBXY * P] = o.sxy;
+    w[S_SBYY * P] = o.syy;
+    w[S_SMB * P] = o.smb;
+    w[S_GTX * P] = o.gtx;
+    w[S_GTY * P] = o.gty;
+    w[S_GBX * P] = o.gbx;
+    w[S_GBY * P] = o.gby;
+    w[S_QSM * P] = o.qsm;
+    w[S_PHI * P] = o.phi;
+    w[S_TMH * P] = o.tmh;
+    w[S_TMB * P] = o.tmb;
+}
+
+// a^alpha b^(1 - alpha) of the mixed forms.  HALF: alpha = 1/2, as one square
+// root: eight pow were most of a node's work (64 x 256 on a B200: the part took 9.5 us of a
+// 34 us step; with this, the unrolled windows and two kernels fewer a step takes 8.7).
+template <bool HALF>
+__device__ __forceinline__ double sgs_mix(double a, double b, double ae) {
+    if constexpr (HALF)
+        return sqrt(a * b);
+    else
+        return pow(a, ae) * pow(b, 1.0 - ae);
+}
+
+// The second part: mixed forms, Germano tensors, Lilly numerators and
+// denominators of a node.
+template <bool HALF>
+__device__ __forceinline__ void sgs_node_c(const SgsB& o, double qbar_h, double phibar_h, const SgsParams& sp,
+                                           double* __restrict__ w, long long P) {
     const double ae = sp.alpha_exp, dx = 1.0, dtest = sp.dtest, delta_t = 1.0;
-    const double nu_mix_t = pow(dtest * dtest * W[S_SMB * P + k], ae) * pow(dtest * qbar_h, 1.0 - ae);
-    const double nu_mix_g = pow(dx * dx * W[S_SMH * P + k], ae) * pow(dx * W[S_QSM * P + k], 1.0 - ae);
+    const double nu_mix_t = sgs_mix<HALF>(dtest * dtest * o.smb, dtest * qbar_h, ae);
+    const double nu_mix_g = sgs_mix<HALF>(dx * dx * o.smh, dx * o.qsm, ae);
     const double kap_mix_t =
-        pow(dtest * dtest * dtest / delta_t * W[S_TMB * P + k], ae) * pow(dtest / delta_t * phibar_h, 1.0 - ae);
-    const double kap_mix_g =
-        pow(dx * dx * dx / delta_t * W[S_TMH * P + k], ae) * pow(dx / delta_t * W[S_PHI * P + k], 1.0 - ae);
-    const double mxx = nu_mix_t * W[S_SBXX * P + k] - nu_mix_g * W[S_SHXX * P + k];
-    const double mxy = nu_mix_t * W[S_SBXY * P + k] - nu_mix_g * W[S_SHXY * P + k];
-    const double myy = nu_mix_t * W[S_SBYY * P + k] - nu_mix_g * W[S_SHYY * P + k];
-    const double mx = kap_mix_t * W[S_GBX * P + k] - kap_mix_g * W[S_GTX * P + k];
-    const double my = kap_mix_t * W[S_GBY * P + k] - kap_mix_g * W[S_GTY * P + k];
-    const double ubx = W[S_UBX * P + k], uby = W[S_UBY * P + k], tb = W[S_TB * P + k];
-    const double lxx = W[S_LXX * P + k] - ubx * ubx;
-    const double lxy = W[S_LXY * P + k] - ubx * uby;
-    const double lyy = W[S_LYY * P + k] - uby * uby;
+        sgs_mix<HALF>(dtest * dtest * dtest / delta_t * o.tmb, dtest / delta_t * phibar_h, ae);
+    const double kap_mix_g = sgs_mix<HALF>(dx * dx * dx / delta_t * o.tmh, dx / delta_t * o.phi, ae);
+    const double mxx = nu_mix_t * o.sxx - nu_mix_g * o.shxx;
+    const double mxy = nu_mix_t * o.sxy - nu_mix_g * o.shxy;
+    const double myy = nu_mix_t * o.syy - nu_mix_g * o.shyy;
+    const double mx = kap_mix_t * o.gbx - kap_mix_g * o.gtx;
+    const double my = kap_mix_t * o.gby - kap_mix_g * o.gty;
+    const double lxx = o.l[0] - o.ubx * o.ubx;
+    const double lxy = o.l[1] - o.ubx * o.uby;
+    const double lyy = o.l[2] - o.uby * o.uby;
     const double lkk3 = (lxx + lyy) / 3.0;
     const double ldxx = lxx - lkk3, ldyy = lyy - lkk3;
-    const double ljx = W[S_LTX * P + k] - ubx * tb;
-    const double ljy = W[S_LTY * P + k] - uby * tb;
-    W[S_NUMV * P + k] = ldxx * mxx + 2.0 * lxy * mxy + ldyy * myy;
-    W[S_DENV * P + k] = mxx * mxx + 2.0 * mxy * mxy + myy * myy;
-    W[S_NUMK * P + k] = ljx * mx + ljy * my;
-    W[S_DENK * P + k] = mx * mx + my * my;
-    W[S_NUMIX * P + k] = nu_mix_g;
-    W[S_KAPMIX * P + k] = kap_mix_g;
+    const double ljx = o.l[3] - o.ubx * o.tb;
+    const double ljy = o.l[4] - o.uby * o.tb;
+    w[S_NUMV * P] = ldxx * mxx + 2.0 * lxy * mxy + ldyy * myy;
+    w[S_DENV * P] = mxx * mxx + 2.0 * mxy * mxy + myy * myy;
+    w[S_NUMK * P] = ljx * mx + ljy * my;
+    w[S_DENK * P] = mx * mx + my * my;
+    w[S_NUMIX * P] = nu_mix_g;
+    w[S_KAPMIX * P] = kap_mix_g;
 }
 
-template <class St>
-__global__ void __launch_bounds__(128) k_sgs_d(SgsGrids<St> S, Geom G, SgsParams sp) {
-    using A = typename Fmt<St>::A;
+// Box of plane p at a node, in window order.
+template <int WIDTH>
+__device__ __forceinline__ double sgs_box(const double* __restrict__ p, const Geom& G, int ix, int iy, int width) {
+    if constexpr (WIDTH == 2) {
+        const bool vx = ix + 1 < G.nx, vy = iy + 1 < G.ny;
+        const int kx = vx ? 1 : 0, ky = vy ? G.pitch : 0;
+        const double* __restrict__ w = p + (iy * G.pitch + ix);
+        const double a = w[0], b = w[kx], c = w[ky], d = w[kx + ky];
+        const double s = ((a + (vx ? b : 0.0)) + (vy ? c : 0.0)) + (vx && vy ? d : 0.0);
+        return s * ((vx ? 0.5 : 1.0) * (vy ? 0.5 : 1.0));
+    } else {
+        const Window w = box_window(G, ix, iy, width);
+        double s = 0.0;
+        for (int yy = w.y0; yy < w.y1; ++yy)
+            for (int xx = w.x0; xx < w.x1; ++xx) s += p[yy * G.pitch + xx];
+        return s / w.cnt;
+    }
+}
+
+template <class St, int WIDTH, bool HALF>
+__global__ void __launch_bounds__(128) k_sgs_c(SgsGrids<St> S, Geom G, SgsParams sp) {
+    pdl_wait();
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ix >= G.nx || iy >= G.ny) return;
-    double* __restrict__ W = S.g[blockIdx.z].W;
-    A* __restrict__ nut_pre = S.g[blockIdx.z].nut;
-    A* __restrict__ at_pre = S.g[blockIdx.z].at;
+    double* __restrict__ W = S.at(blockIdx.z).W;
+    const long long P = G.plane;
+    double* __restrict__ w = W + iy * G.pitch + ix;
+    SgsB o;
+    o.ubx = w[S_UBX * P];
+    o.uby = w[S_UBY * P];
+    o.tb = w[S_TB * P];
+#pragma unroll
+    for (int p = 0; p < 5; ++p) o.l[p] = w[(S_LXX + p) * P];
+    o.shxx = w[S_SHXX * P];
+    o.shxy = w[S_SHXY * P];
+    o.shyy = w[S_SHYY * P];
+    o.smh = w[S_SMH * P];
+    o.sxx = w[S_SBXX * P];
+    o.sxy = w[S_SBXY * P];
+    o.syy = w[S_SBYY * P];
+    o.smb = w[S_SMB * P];
+    o.gtx = w[S_GTX * P];
+    o.gty = w[S_GTY * P];
+    o.gbx = w[S_GBX * P];
+    o.gby = w[S_GBY * P];
+    o.qsm = w[S_QSM * P];
+    o.phi = w[S_PHI * P];
+    o.tmh = w[S_TMH * P];
+    o.tmb = w[S_TMB * P];
+    const double qbar_h = sgs_box<WIDTH>(W + S_QSM * P, G, ix, iy, sp.width);
+    const double phibar_h = sgs_box<WIDTH>(W + S_PHI * P, G, ix, iy, sp.width);
+    sgs_node_c<HALF>(o, qbar_h, phibar_h, sp, w, P);
+}
+
+// k_sgs_b and k_sgs_c in one for the test filter of two nodes: a node forms
+// qsm^1/2 and Phi_sm^1/2 of its window itself (three more square roots), so only
+// the six results go through memory and one launch is saved.
+template <class St, bool HALF>
+__global__ void __launch_bounds__(128) k_sgs_bc2(SgsGrids<St> S, Geom G, SgsParams sp) {
+    pdl_wait();
+    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
+    const int iy = blockIdx.y * blockDim.y + threadIdx.y;
+    if (ix >= G.nx || iy >= G.ny) return;
+    const SgsGrid<St> io = S.at(blockIdx.z);
+    SgsB o;
+    double qbar_h, phibar_h;
+    sgs_node_b2<St, true>(io, G, ix, iy, sp, o, qbar_h, phibar_h);
+    sgs_node_c<HALF>(o, qbar_h, phibar_h, sp, io.W + iy * G.pitch + ix, G.plane);
+}
+
+// The third part of a node: regularised Lilly coefficients, nu_t and alpha_t.
+template <int WIDTH>
+__device__ __forceinline__ void sgs_node_d(double* __restrict__ W, const Geom& G, int ix, int iy, const SgsParams& sp,
+                                           double& nut, double& at_out) {
     const long long P = G.plane;
     const int k = iy * G.pitch + ix;
-    const Window w = box_window(G, ix, iy, sp.width);
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int yy = w.y0; yy < w.y1; ++yy)
-        for (int xx = w.x0; xx < w.x1; ++xx) {
-            const int kk = yy * G.pitch + xx;
+    double s[4];
 #pragma unroll
-            for (int p = 0; p < 4; ++p) s[p] += W[(S_NUMV + p) * P + kk];
-        }
-    const double cnu = lilly_coefficient(s[0] / w.cnt, s[1] / w.cnt);
-    const double ck = lilly_coefficient(s[2] / w.cnt, s[3] / w.cnt);
+    for (int p = 0; p < 4; ++p) s[p] = sgs_box<WIDTH>(W + (S_NUMV + p) * P, G, ix, iy, sp.width);
+    const double cnu = lilly_coefficient(s[0], s[1]);
+    const double ck = lilly_coefficient(s[2], s[3]);
     W[S_CNU * P + k] = cnu;
     W[S_CK * P + k] = ck;
     const double margin = (TAU_TRT_FLOOR - 0.5) / 3.0;
     const double nt = cnu * W[S_NUMIX * P + k];
     const double nu_t_min = fmax(sp.nu_sm_min * sp.nu_mol, margin - sp.nu_mol);
-    nut_pre[k] = A(nt < nu_t_min ? nu_t_min : nt);
+    nut = nt < nu_t_min ? nu_t_min : nt;
     const double at = ck * W[S_KAPMIX * P + k];
     const double alpha_t_min = fmax(sp.nu_sm_min * sp.alpha_mol, margin - sp.alpha_mol);
-    at_pre[k] = A(at < alpha_t_min ? alpha_t_min : at);
+    at_out = at < alpha_t_min ? alpha_t_min : at;
+}
+
+template <class St, int WIDTH>
+__global__ void __launch_bounds__(128) k_sgs_d(SgsGrids<St> S, Geom G, SgsParams sp) {
+    using A = typename Fmt<St>::A;
+    pdl_wait();
+    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
+    const int iy = blockIdx.y * blockDim.y + threadIdx.y;
+    if (ix >= G.nx || iy >= G.ny) return;
+    const SgsGrid<St> io = S.at(blockIdx.z);
+    const int k = iy * G.pitch + ix;
+    double nut, at;
+    sgs_node_d<WIDTH>(io.W, G, ix, iy, sp, nut, at);
+    io.nut[k] = A(nut);
+    io.at[k] = A(at);
+}
+
+// The last part of the model (width 2) and the collision of the node that it is for
+// (k_collide_ref with the node's nu_t / alpha_t).
+template <class St>
+__global__ void __launch_bounds__(128) k_sgs_collide2(const St* __restrict__ src, St* __restrict__ dst,
+                                                      const typename Fmt<St>::A* __restrict__ rho,
+                                                      const typename Fmt<St>::A* __restrict__ ux,
+                                                      const typename Fmt<St>::A* __restrict__ uy,
+                                                      const typename Fmt<St>::A* __restrict__ tt,
+                                                      typename Fmt<St>::A* __restrict__ fy,
+                                                      typename Fmt<St>::A* __restrict__ nut, double* __restrict__ W,
+                                                      Geom G, SgsParams sp, StepScalars<typename Fmt<St>::A> c) {
+    using A = typename Fmt<St>::A;
+    pdl_wait();
+    const int ix = blockIdx.x * blockDim.x + threadIdx.x;
+    const int iy = blockIdx.y * blockDim.y + threadIdx.y;
+    if (ix >= G.nx || iy >= G.ny) return;
+    double nt, at;
+    sgs_node_d<2>(W, G, ix, iy, sp, nt, at);
+    const A nt_a = A(nt), at_a = A(at);
+    collide_ref_node<St>(src, dst, rho, ux, uy, tt, fy, nut, G, ix, iy, c, &nt_a, &at_a);
 }
 
 // Mean and max of the Lilly coefficients (cs_dyn_mean / _max, kappa_dyn_mean

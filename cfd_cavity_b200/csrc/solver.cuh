@@ -196,6 +196,7 @@ struct Impl final : Solver {
     bool sgs_valid = false;        // the work planes hold the last step's coefficients
 
     ~Impl() override {
+        drop_dyn_graphs();
         for (auto& row : graph)
             for (auto& gx : row)
                 if (gx) cudaGraphExecDestroy(gx);
@@ -519,6 +520,8 @@ struct Impl final : Solver {
             CK(cudaMalloc(&sgs_out, sizeof(double) * 4));
         }
         sgs_valid = false;
+        CK(cudaStreamSynchronize(stream));
+        drop_dyn_graphs();  // the model's constants are in their launches
     }
 
     void dynamic_stats(double* out4) override {
@@ -535,12 +538,16 @@ struct Impl final : Solver {
     // One step with the dynamic model, in the reference's order
     // (src/uniform/solver.rs:279-291): compute_dynamic_sgs on the REF state,
     // collide with the per-node nu_t / alpha_t, then stream + BC + macro +
-    // no-slip back to a REF state.
-    void dyn_step() {
-        to_ref_form();
+    // no-slip back to a REF state (in the buffer it came from).  The step
+    // index of the rounding is s, or *sdev + s in graph replays.
+    void launch_dyn(int64_t s, const long long* sdev) {
+        const int64_t ramp_s = sdev ? spin_up : s;
+        StepScalars<A> c = scalars(ramp_s);
+        c.step = s;
+        c.step_dev = sdev;
         double nu_eff = U.nu;
-        if (time_step < spin_up) {
-            const double x = double(time_step) / double(spin_up);
+        if (ramp_s < spin_up) {
+            const double x = double(ramp_s) / double(spin_up);
             const double nu_start = U.nu * nu_start_mult;
             nu_eff = nu_start * std::pow(U.nu / nu_start, x);
         }
@@ -555,32 +562,91 @@ struct Impl final : Solver {
         sp.nu_sm_min = dyn_min;
         SgsGrids<St> S{};
         S.g[0] = SgsGrid<St>{pop[cur], rho, ux, uy, tt, sgs_w, nut_pre, at_pre};
-        k_sgs_b<St><<<grd, blk, 0, stream>>>(S, G, sp);
+        const St* src = pop[cur];
+        St* dst = pop[cur ^ 1];
+        if (sp.width == 2) {
+            if (sp.alpha_exp == 0.5)
+                launch_pdl(k_sgs_bc2<St, true>, stream, S, G, sp);
+            else
+                launch_pdl(k_sgs_bc2<St, false>, stream, S, G, sp);
+            check_launch();
+            launch_pdl(k_sgs_collide2<St>, stream, src, dst, (const A*)rho, (const A*)ux, (const A*)uy, (const A*)tt,
+                       fy, nut, sgs_w, G, sp, c);
+            check_launch();
+        } else {
+            launch_pdl(k_sgs_b<St, 0>, stream, S, G, sp);
+            check_launch();
+            launch_pdl(sp.alpha_exp == 0.5 ? k_sgs_c<St, 0, true> : k_sgs_c<St, 0, false>, stream, S, G, sp);
+            check_launch();
+            launch_pdl(k_sgs_d<St, 0>, stream, S, G, sp);
+            check_launch();
+            launch_pdl(k_collide_ref<St>, stream, src, dst, (const A*)rho, (const A*)ux, (const A*)uy, (const A*)tt,
+                       fy, nut, G, c, (const A*)nut_pre, (const A*)at_pre);
+            check_launch();
+        }
+        launch_pdl(k_materialize<St, false>, stream, (const St*)dst, pop[cur], (const A*)fy, rho, ux, uy, tt, G, c);
         check_launch();
-        k_sgs_c<St><<<grd, blk, 0, stream>>>(S, G, sp);
-        check_launch();
-        k_sgs_d<St><<<grd, blk, 0, stream>>>(S, G, sp);
-        check_launch();
-        sgs_valid = true;
-        k_collide_ref<St><<<grd, blk, 0, stream>>>(pop[cur], pop[cur ^ 1], rho, ux, uy, tt, fy, nut, G,
-                                                   scalars(time_step), nut_pre, at_pre);
-        check_launch();
-        cur ^= 1;
-        pc_form = true;
-        ref_cached = false;
-        to_ref_form();
-        time_step += 1;
         if (acc_on) {
             k_acc_nu_ref<A><<<(p.ny + 127) / 128, 128, 0, stream>>>(tt, acc_hot, acc_cold, G);
             check_launch();
-            n_acc += 1;
         }
+    }
+
+    // DYN_GRAPH_STEPS steady-state steps with the dynamic model as one graph.
+    static constexpr int DYN_GRAPH_STEPS = 16;
+    cudaGraphExec_t dgraph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+    int64_t dgraph_launches[2][2] = {{0, 0}, {0, 0}};
+    void drop_dyn_graphs() {
+        for (auto& row : dgraph)
+            for (auto& gx : row)
+                if (gx) {
+                    cudaGraphExecDestroy(gx);
+                    gx = nullptr;
+                }
+    }
+    void replay_dyn() {
+        cudaGraphExec_t& gx = dgraph[cur][acc_on ? 1 : 0];
+        int64_t& nl = dgraph_launches[cur][acc_on ? 1 : 0];
+        const int64_t l0 = launches;
+        if (!gx) {
+            CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+            for (int j = 0; j < DYN_GRAPH_STEPS; ++j) launch_dyn(j, step_dev);
+            k_add_step<<<1, 1, 0, stream>>>(step_dev, DYN_GRAPH_STEPS);
+            cudaGraph_t gr;
+            CK(cudaStreamEndCapture(stream, &gr));
+            nl = launches - l0 + 1;
+            CK(cudaGraphInstantiate(&gx, gr, 0));
+            cudaGraphDestroy(gr);
+        }
+        if (step_dev_val != time_step) {
+            k_set_step<<<1, 1, 0, stream>>>(step_dev, time_step);
+            CK(cudaGetLastError());
+            step_dev_val = time_step;
+        }
+        CK(cudaGraphLaunch(gx, stream));
+        launches = l0 + nl;
+        step_dev_val += DYN_GRAPH_STEPS;
+    }
+
+    void step_dyn(int64_t n) {
+        to_ref_form();
+        if (acc_on) n_acc += n;
+        while (n > 0) {
+            const int64_t k = n >= DYN_GRAPH_STEPS && time_step >= spin_up ? DYN_GRAPH_STEPS : 1;
+            if (k > 1)
+                replay_dyn();
+            else
+                launch_dyn(time_step, nullptr);
+            time_step += k;
+            n -= k;
+        }
+        sgs_valid = true;
     }
 
     void step(int64_t n) override {
         if (n <= 0) return;
         if (dyn) {
-            for (int64_t j = 0; j < n; ++j) dyn_step();
+            step_dyn(n);
             return;
         }
         bool first = true;
