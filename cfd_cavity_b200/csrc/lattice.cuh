@@ -383,6 +383,64 @@ CAV_OVER(over_2cs4, 0.5, I4H, I4L, A(2.0) * A(CS2) * A(CS2))
 #undef CAV_OVER
 
 // ---------------------------------------------------------------------------
+// FP64 quotients without a branch, rounded like `/`.  1/b by Newton steps from the
+// special-function unit's approximation (relative error below 2^-19): y1 = y0
+// (1 + e + e^2) is within 0.57 ulp, y2 = RN(y1 + y1 RN(1 - b y1)) the rounded
+// reciprocal but for a significand of all ones (1 - 2^-53, an ordinary density):
+// there 1/b lies just above the middle of 2^k and its successor and is the
+// successor, the odd one; a / b by two remainder corrections of a y, r = a - b q exact and
+// q = RN(q + r y) -- Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990, theorems on the
+// rounded reciprocal and quotient.  For b and a / b away from the ends of the
+// exponent range: here b is a density, a relaxation time or a fixed ratio of
+// order one; a numerator below 2^-900 may lose its last bit.  Infinite and NaN
+// quotients come out as a * y.  Checked against the division itself on 2^28
+// operand pairs (tests/test_gpu_quotient.py).  A compiled division checks its
+// range and branches, and code does not move across it.  B200, us per step with
+// divisions / with these: FP64 16 x 40 2.36 / 2.03, 64 x 256 2.54 / 2.16, 128 x 511
+// 4.52 / 4.30, the dynamic model on 64 x 256 8.52 / 8.02; the block-refined 64 x 256 in
+// three levels 40.3 / 37.2 per coarse step.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ double rcp_rn(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = __fma_rn(-b, y, 1.0);
+    y = __fma_rn(y, __fma_rn(e, e, e), y);
+    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    const bool ones = __double2loint(b) == -1 && (__double2hiint(b) | int(0xfff00000u)) == -1;
+    return __hiloint2double(__double2hiint(y), __double2loint(y) | (ones ? 1 : 0));
+}
+// a / b from y = rcp_rn(b) (or the host's rounded 1 / b)
+__device__ __forceinline__ double quot_rn(double a, double b, double y) {
+    const double q0 = __dmul_rn(a, y);
+    const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+    const double q2 = __fma_rn(__fma_rn(-b, q1, a), y, q1);
+    return isfinite(q0) ? q2 : q0;
+}
+
+// sqrt(x) without a branch: Newton steps on g = x y and h = y / 2 from the
+// special-function unit's y ~ 1 / sqrt(x) (Goldschmidt's coupled iteration as
+// in Markstein, above), then one exact-remainder correction, g + (x - g^2) h:
+// rounded as sqrt() but for the few x per binade whose root lies within
+// 2^-53 ulp of the middle of two numbers.  Zero, infinite and NaN x, and x below
+// 2^-960, come back as they are.  For the dynamic model's dozen independent roots
+// (64 x 256: 8.02 -> 7.52 us per step); the step itself has one, at the end of a
+// chain, where sqrt() is the shorter (2.05 us against 2.26 on 16 x 40).
+__device__ __forceinline__ double sqrt_nr(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double g = __dmul_rn(x, y), h = __dmul_rn(0.5, y);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const double r = __fma_rn(-g, h, 0.5);
+        g = __fma_rn(g, r, g);
+        h = __fma_rn(h, r, h);
+    }
+    g = __fma_rn(__fma_rn(-g, g, x), h, g);
+    return x >= 0x1p-960 && x <= 0x1p960 ? g : x;
+}
+
+// ---------------------------------------------------------------------------
 // Equilibria.  In the unshifted (FP64) form the expressions are those of the
 // reference (feq form restated at src/uniform/tests.rs:314-316), its divisions
 // by cs^2 and cs^4 in the form above; the shifted form returns feq_i - w_i
@@ -544,9 +602,10 @@ __device__ __forceinline__ Macro<A, SHIFT> macro_f(const A (&f)[Q], A fy_prev, b
         m.drho = s - A(1.0);
         m.inv_rho = A(0.0);
         if (r > A(2.220446049250313e-16)) {
-            un = un / r;
-            vn = vn / r;
-            vn = vn + A(0.5) * fy_prev / r;
+            const A y = rcp_rn(r);
+            un = quot_rn(un, r, y);
+            vn = quot_rn(vn, r, y);
+            vn = vn + quot_rn(A(0.5) * fy_prev, r, y);
         }
         m.rho = r;
         m.ux = wall ? A(0.0) : un;
@@ -758,13 +817,15 @@ __device__ __forceinline__ CollF<A> collide_f_pre(const A (&f)[Q], const Macro<A
         double pyy = ((((d_f[2] + d_f[3]) + d_f[4]) + d_f[6]) + d_f[7]) + d_f[8];
         double pi2 = pxx * pxx + 2.0 * pxy * pxy + pyy * pyy;
         double rho_m = r > 1e-12 ? r : 1e-12;
-        double s_mag = sqrt(pi2) / (2.0 * CS2 * c.tau_s * rho_m);
+        const double den = 2.0 * CS2 * c.tau_s * rho_m;
+        double s_mag = quot_rn(sqrt(pi2), den, rcp_rn(den));
         double nut = nut_ovr ? double(*nut_ovr) : c.cs * c.cs * s_mag;
         o.nut = nut;
         double tau_plus = 0.5 + 3.0 * (c.nu + nut);
-        double tau_minus = 0.5 + LAMBDA_TRT / (tau_plus - 0.5);
+        const double t_half = tau_plus - 0.5;
+        double tau_minus = 0.5 + quot_rn(LAMBDA_TRT, t_half, rcp_rn(t_half));
         // (0.5 / tau is 0.5 times the rounded 1 / tau)
-        const double inv_p = 1.0 / tau_plus, inv_m = 1.0 / tau_minus;
+        const double inv_p = rcp_rn(tau_plus), inv_m = rcp_rn(tau_minus);
         o.w1 = 0.5 * (inv_p + inv_m);
         o.w2 = 0.5 * (inv_p - inv_m);
         o.k1 = 1.0 - 0.5 * inv_m;
@@ -808,11 +869,11 @@ __device__ __forceinline__ void collide_g(A (&g)[Q], A temp, A u, A v, A nut, co
         double d_g[Q];
 #pragma unroll
         for (int i = 0; i < Q; ++i) d_g[i] = g[i] - geq_full<double>(i, temp, u, v, c.geq_order);
-        double alpha_t = at_ovr ? double(*at_ovr) : nut / c.pr_t;
-        double tau_t_plus = 0.5 + 3.0 * (c.alpha + alpha_t);
-        double tau_t_minus = tau_t_plus;
-        double a_g = 0.5 * (1.0 / tau_t_plus + 1.0 / tau_t_minus);
-        double b_g = 0.5 * (1.0 / tau_t_plus - 1.0 / tau_t_minus);
+        double alpha_t = at_ovr ? double(*at_ovr) : quot_rn(nut, c.pr_t, c.inv_pr_t);
+        double tau_t = 0.5 + 3.0 * (c.alpha + alpha_t);  // tau_t- = tau_t+
+        const double inv_t = rcp_rn(tau_t);
+        double a_g = 0.5 * (inv_t + inv_t);
+        double b_g = 0.5 * (inv_t - inv_t);
 #pragma unroll
         for (int i = 0; i < Q; ++i) g[i] = g[i] + (-a_g * d_g[i] - b_g * d_g[OPP(i)]);
     } else {

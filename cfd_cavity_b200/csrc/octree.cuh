@@ -173,6 +173,14 @@ __device__ __forceinline__ void oct_collide_g_sh(float (&g)[Q], float u, float v
     }
 }
 
+// 1 / b and a / b of the level arithmetic (FP64 without a branch).
+__device__ __forceinline__ double oct_inv(double b) { return rcp_rn(b); }
+__device__ __forceinline__ float oct_inv(float b) { return 1.0f / b; }
+__device__ __forceinline__ double oct_div(double a, double b) { return quot_rn(a, b, rcp_rn(b)); }
+__device__ __forceinline__ float oct_div(float a, float b) { return a / b; }
+__device__ __forceinline__ double oct_third(double a) { return quot_rn(a, 3.0, 1.0 / 3.0); }
+__device__ __forceinline__ float oct_third(float a) { return a / 3.0f; }
+
 template <class A, bool SHIFT>
 __device__ __forceinline__ void oct_collide(A (&f)[Q], A (&g)[Q], const Macro<A, SHIFT>& m, const LvlScal<A>& c0,
                                             A& fy_out, const A* nut = nullptr, const A* at = nullptr) {
@@ -180,17 +188,18 @@ __device__ __forceinline__ void oct_collide(A (&f)[Q], A (&g)[Q], const Macro<A,
     if (nut) {
         // dynamic model: relaxation times rebuilt per node from the level's
         // tau and the node's nu_t / alpha_t (src/octree/cavity.rs:100-110)
-        const A tp = A(0.5) + A(3.0) * (c0.tp - A(0.5)) / A(3.0) + A(3.0) * *nut;
-        const A tm = A(0.5) + A(LAMBDA_TRT) / (tp - A(0.5));
-        const A tt = A(0.5) + A(3.0) * (c0.tt - A(0.5)) / A(3.0) + A(3.0) * *at;
-        c.a_f = A(0.5) * (A(1.0) / tp + A(1.0) / tm);
-        c.b_f = A(0.5) * (A(1.0) / tp - A(1.0) / tm);
-        c.a_g = A(1.0) / tt;
-        c.c_m = A(1.0) - A(0.5) / tm;
-        c.c_p = A(1.0) - A(0.5) / tp;
-        c.om_p = A(1.0) / tp;
-        c.om_m = A(1.0) / tm;
-        c.om_g = A(1.0) / tt;
+        const A tp = A(0.5) + oct_third(A(3.0) * (c0.tp - A(0.5))) + A(3.0) * *nut;
+        const A tm = A(0.5) + oct_div(A(LAMBDA_TRT), tp - A(0.5));
+        const A tt = A(0.5) + oct_third(A(3.0) * (c0.tt - A(0.5))) + A(3.0) * *at;
+        // (0.5 / tau is 0.5 times the rounded 1 / tau)
+        c.om_p = oct_inv(tp);
+        c.om_m = oct_inv(tm);
+        c.om_g = oct_inv(tt);
+        c.a_f = A(0.5) * (c.om_p + c.om_m);
+        c.b_f = A(0.5) * (c.om_p - c.om_m);
+        c.a_g = c.om_g;
+        c.c_m = A(1.0) - A(0.5) * c.om_m;
+        c.c_p = A(1.0) - A(0.5) * c.om_p;
         c.k_p = c.c_p;
         c.k_m = c.c_m;
         c.cs = A(0.0);
@@ -639,7 +648,7 @@ __global__ void __launch_bounds__(OT) k_oct_collide(LvlPair<St> P, const OctScal
     m.ux = L.mac[L.n + k];
     m.uy = L.mac[2 * L.n + k];
     m.t = L.mac[3 * L.n + k];
-    m.inv_rho = A(1.0) / m.rho;
+    m.inv_rho = oct_inv(m.rho);
     const A* nut = blockIdx.y == 0 ? D.nut[0] : D.nut[1];
     const A* at = blockIdx.y == 0 ? D.at[0] : D.at[1];
     A fy_new;
@@ -673,11 +682,15 @@ __device__ __forceinline__ Macro<A, SHIFT> refresh(const A (&f)[Q], const A (&g)
     if (GUARD && !(m.rho > A(2.220446049250313e-16))) {
         m.ux = A(0.0);
         m.uy = A(0.0);
-    } else {
+    } else if constexpr (SHIFT) {
         m.ux = mx / m.rho;
         m.uy = my / m.rho;
+    } else {
+        const A y = rcp_rn(m.rho);
+        m.ux = quot_rn(mx, m.rho, y);
+        m.uy = quot_rn(my, m.rho, y);
     }
-    m.inv_rho = A(1.0) / m.rho;
+    m.inv_rho = oct_inv(m.rho);
     return m;
 }
 
@@ -694,7 +707,7 @@ __device__ __forceinline__ void rescale(const A (&fn)[Q], const Xi<A>& xi, A (&o
         else if constexpr (SHIFT)
             out[i] = even * xi.inv_even + odd * xi.inv_odd;
         else
-            out[i] = even / xi.even + odd / xi.odd;
+            out[i] = quot_rn(even, xi.even, xi.inv_even) + quot_rn(odd, xi.odd, xi.inv_odd);
     }
 }
 
@@ -856,7 +869,7 @@ __global__ void __launch_bounds__(OT) k_oct_f2c(LvlPair<StF> F, LvlPair<StC> C, 
         if constexpr (SH)
             g[i] = geq_full<A>(i, tt, ux, uy, 2) + c[13 + i] * xi.inv_th;
         else
-            g[i] = geq_full<A>(i, tt, ux, uy, 2) + c[13 + i] / xi.th;
+            g[i] = geq_full<A>(i, tt, ux, uy, 2) + quot_rn(c[13 + i], xi.th, xi.inv_th);
     }
     store_pops<StC, true>(Lc.ref_out, Lc.n, e.kc, f, g, true, seed, sidx * 16 + phase, (long long)Lc.node_off + e.kc);
     const Macro<A, SH> m = refresh<A, SH, true>(f, g);

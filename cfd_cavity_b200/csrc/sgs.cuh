@@ -158,17 +158,18 @@ __device__ __forceinline__ void sgs_strain(const SgsGrid<St>& io, const Geom& G,
     const double rho_m = rho_k > 1e-12 ? rho_k : 1e-12;
     const double denom = 2.0 * CS2 * sp.tau_s * rho_m;
     const double pi2 = pi_xx * pi_xx + 2.0 * pi_xy * pi_xy + pi_yy * pi_yy;
-    o.shxx = -pi_xx / denom;
-    o.shxy = -pi_xy / denom;
-    o.shyy = -pi_yy / denom;
-    o.smh = sqrt(pi2) / denom;
+    const double inv = rcp_rn(denom);
+    o.shxx = quot_rn(-pi_xx, denom, inv);
+    o.shxy = quot_rn(-pi_xy, denom, inv);
+    o.shyy = quot_rn(-pi_yy, denom, inv);
+    o.smh = quot_rn(sqrt_nr(pi2), denom, inv);
 }
 
 // qsm^1/2 and Phi_sm^1/2 of a node from its fields and boxes.
 __device__ __forceinline__ void sgs_small(double u, double v, double t, double ub, double vb, double tb, double& q,
                                           double& phi) {
     const double du = u - ub, dv = v - vb;
-    const double r = sqrt(0.5 * (du * du + dv * dv));
+    const double r = sqrt_nr(0.5 * (du * du + dv * dv));
     q = r / 2.0;
     phi = 0.5 * fabs(t - tb) * r;
 }
@@ -177,10 +178,10 @@ __device__ __forceinline__ void sgs_small(double u, double v, double t, double u
 __device__ __forceinline__ void sgs_flux(SgsB& o) {
     const double th_x = o.gtx * o.shxx + o.gty * o.shxy;
     const double th_y = o.gtx * o.shxy + o.gty * o.shyy;
-    o.tmh = sqrt(2.0 * (th_x * th_x + th_y * th_y));
+    o.tmh = sqrt_nr(2.0 * (th_x * th_x + th_y * th_y));
     const double tb_x = o.gbx * o.sxx + o.gby * o.sxy;
     const double tb_y = o.gbx * o.sxy + o.gby * o.syy;
-    o.tmb = sqrt(2.0 * (tb_x * tb_x + tb_y * tb_y));
+    o.tmb = sqrt_nr(2.0 * (tb_x * tb_x + tb_y * tb_y));
 }
 
 // The first part for any test-filter width.
@@ -222,7 +223,7 @@ __device__ __forceinline__ void sgs_node_b(const SgsGrid<St>& io, const Geom& G,
     o.sxx = 0.5 * (ubx_xp - ubx_xm);
     o.syy = 0.5 * (uby_yp - uby_ym);
     o.sxy = 0.5 * (0.5 * (uby_xp - uby_xm) + 0.5 * (ubx_yp - ubx_ym));
-    o.smb = sqrt(o.sxx * o.sxx + 2.0 * o.sxy * o.sxy + o.syy * o.syy);
+    o.smb = sqrt_nr(o.sxx * o.sxx + 2.0 * o.sxy * o.sxy + o.syy * o.syy);
     o.gtx = ddx_f(tt, G, ix, iy);
     o.gty = ddy_f(tt, G, ix, iy);
     o.gbx = 0.5 * (tb_xp - tb_xm);
@@ -299,7 +300,7 @@ __device__ __forceinline__ void sgs_node_b2(const SgsGrid<St>& io, const Geom& G
     o.sxx = 0.5 * (bu.e - bu.w);
     o.syy = 0.5 * (bv.n - bv.s);
     o.sxy = 0.5 * (0.5 * (bv.e - bv.w) + 0.5 * (bu.n - bu.s));
-    o.smb = sqrt(o.sxx * o.sxx + 2.0 * o.sxy * o.sxy + o.syy * o.syy);
+    o.smb = sqrt_nr(o.sxx * o.sxx + 2.0 * o.sxy * o.sxy + o.syy * o.syy);
     o.gtx = 0.5 * ((x1 ? tv[1][2] : t_k) - (x0 ? t_k : tv[1][0]));
     o.gty = 0.5 * ((y1 ? tv[2][1] : t_k) - (y0 ? t_k : tv[0][1]));
     o.gbx = 0.5 * (bt.e - bt.w);
@@ -357,11 +358,11 @@ __global__ void __launch_bounds__(128) k_sgs_b(SgsGrids<St> S, Geom G, SgsParams
 
 // a^alpha b^(1 - alpha) of the mixed forms.  HALF: alpha = 1/2, as one square
 // root: eight pow were most of a node's work (64 x 256 on a B200: the part took 9.5 us of a
-// 34 us step; with this, the unrolled windows and two kernels fewer a step takes 8.7).
+// 34 us step; with this, the unrolled windows and two kernels fewer a step took 8.7).
 template <bool HALF>
 __device__ __forceinline__ double sgs_mix(double a, double b, double ae) {
     if constexpr (HALF)
-        return sqrt(a * b);
+        return sqrt_nr(a * b);
     else
         return pow(a, ae) * pow(b, 1.0 - ae);
 }
@@ -385,7 +386,7 @@ __device__ __forceinline__ void sgs_node_c(const SgsB& o, double qbar_h, double 
     const double lxx = o.l[0] - o.ubx * o.ubx;
     const double lxy = o.l[1] - o.ubx * o.uby;
     const double lyy = o.l[2] - o.uby * o.uby;
-    const double lkk3 = (lxx + lyy) / 3.0;
+    const double lkk3 = quot_rn(lxx + lyy, 3.0, 1.0 / 3.0);
     const double ldxx = lxx - lkk3, ldyy = lyy - lkk3;
     const double ljx = o.l[3] - o.ubx * o.tb;
     const double ljy = o.l[4] - o.uby * o.tb;
