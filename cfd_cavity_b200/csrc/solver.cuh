@@ -918,8 +918,8 @@ struct Impl final : Solver {
             if (N < 2 || ws < 1 || ws > N || C < 2) throw ArgError{CAV_ERR_ARG, "bad adjoint spec"};
             const size_t fld = field_elems(), popn = size_t(NPLANES) * fld;
             const int64_t n_ck = (N - 1 + C - 1) / C;
-            St *ck_pop = nullptr, *seg_pop = nullptr;
-            A *ck_fy = nullptr, *seg_fy = nullptr, *P[2] = {nullptr, nullptr};
+            St* ck_pop = nullptr;
+            A *ck_fy = nullptr, *P[2] = {nullptr, nullptr};
             double *acc_cs_d = nullptr, *acc_th_d = nullptr;
             cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
             struct Free {
@@ -935,12 +935,12 @@ struct Impl final : Solver {
             };
             dalloc((void**)&ck_pop, sizeof(St) * popn * n_ck);
             dalloc((void**)&ck_fy, sizeof(A) * fld * n_ck);
-            St* seg_pop2 = nullptr;
-            A* seg_fy2 = nullptr;
-            dalloc((void**)&seg_pop, sizeof(St) * popn * C);
-            dalloc((void**)&seg_fy, sizeof(A) * fld * C);
-            dalloc((void**)&seg_pop2, sizeof(St) * popn * C);
-            dalloc((void**)&seg_fy2, sizeof(A) * fld * C);
+            St* setp[2] = {nullptr, nullptr};
+            A* setf[2] = {nullptr, nullptr};
+            for (int set = 0; set < 2; ++set) {
+                dalloc((void**)&setp[set], sizeof(St) * popn * C);
+                dalloc((void**)&setf[set], sizeof(A) * fld * C);
+            }
             long long* sdev2 = nullptr;
             dalloc((void**)&sdev2, 2 * sizeof(long long));
             for (auto& pp : P) dalloc((void**)&pp, sizeof(A) * APLANES * fld);
@@ -974,6 +974,7 @@ struct Impl final : Solver {
                                    stream));
                 CK(cudaStreamSynchronize(stream));
             }
+            AdjScal<A> sc{table, S, scalars(spin_up)};
             AdjObj<A> obj;
             obj.ws = ws;
             obj.coef = A(U.lz / (double(p.ny) * double(N - ws + 1)));
@@ -982,10 +983,10 @@ struct Impl final : Solver {
             // adjoint sweep of segment k (the solver's stream, set k & 1):
             // both are latency-bound on one cavity, so the GPU runs them side
             // by side.  Events order the reuse of a slot set.  Each stream has
-            // its own device step counter; full segments (length C, even) are
-            // CUDA graphs, one pair per slot set.
-            St* setp[2] = {seg_pop, seg_pop2};
-            A* setf[2] = {seg_fy, seg_fy2};
+            // its own device step counter; full segments (length C, even) past
+            // the ramps are CUDA graphs, one pair per slot set, with the steady
+            // scalars in their launches; the others are launched step by step
+            // with the scalars of the table.
             long long* sd_rec = sdev2;
             long long* sd_adj = sdev2 + 1;
             cudaStream_t rs = nullptr, hs = nullptr;
@@ -1033,41 +1034,55 @@ struct Impl final : Solver {
                 CK(cudaEventCreateWithFlags(&ev_adj[k], cudaEventDisableTiming));
             }
             const bool use_graphs = (C % 2) == 0;
-            auto capture = [&](cudaStream_t st, cudaGraphExec_t* out, auto&& body) {
-                const int64_t l0 = launches;
-                CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+            auto capture = [&](cudaGraphExec_t* out, auto&& body) {
+                CK(cudaStreamBeginCapture(rs, cudaStreamCaptureModeThreadLocal));
                 body();
                 cudaGraph_t gr;
-                CK(cudaStreamEndCapture(st, &gr));
-                launches = l0;
+                CK(cudaStreamEndCapture(rs, &gr));
                 CK(cudaGraphInstantiate(out, gr, 0));
                 cudaGraphDestroy(gr);
+                CK(cudaGraphUpload(*out, rs));
             };
             auto seg_len = [&](int64_t k) { return std::min<int64_t>(1 + k * C + C, N) - (1 + k * C); };
+            auto replayed = [&](int64_t k) { return use_graphs && seg_len(k) == C && 1 + k * C >= spin_up; };
+            // one recomputed step / one reverse step of slot set `set`
+            auto fwd_step = [&](cudaStream_t st, int set, int64_t j, bool steady, const long long* sdev, int64_t s) {
+                const St* src = setp[set] + popn * j;
+                St* dst = setp[set] + popn * (j + 1);
+                const A* fi = setf[set] + fld * j;
+                A* fo = setf[set] + fld * (j + 1);
+                if (steady)
+                    launch_pdl(k_fwd_slot<St, true>, st, src, dst, fi, fo, G, sc, sdev, s);
+                else
+                    launch_pdl(k_fwd_slot<St, false>, st, src, dst, fi, fo, G, sc, sdev, s);
+            };
+            auto adj_step = [&](cudaStream_t st, int set, int64_t j, int q, bool steady, const long long* sdev, int64_t s) {
+                const St* X = setp[set] + popn * j;
+                const A* F = setf[set] + fld * j;
+                const St* Xp = j > 0 ? X - popn : nullptr;
+                const A* Fp = j > 0 ? F - fld : nullptr;
+                if (steady)
+                    launch_pdl(k_adj_step<St, true>, st, X, F, P[q], P[q ^ 1], acc_cs_d, acc_th_d, G, sc, sdev, s, obj, Xp,
+                               Fp);
+                else
+                    launch_pdl(k_adj_step<St, false>, st, X, F, P[q], P[q ^ 1], acc_cs_d, acc_th_d, G, sc, sdev, s, obj,
+                               Xp, Fp);
+            };
             // recomputation of segment k on rs
             auto recompute = [&](int64_t k) {
                 const int set = int(k & 1);
                 const int64_t a = 1 + k * C, L = seg_len(k);
-                St* sp = setp[set];
-                A* sf = setf[set];
                 if (k + 2 < n_ck) CK(cudaStreamWaitEvent(rs, ev_adj[k + 2], 0));  // set free again
-                CK(cudaMemcpyAsync(sp, ck_pop + popn * k, sizeof(St) * popn, cudaMemcpyDeviceToDevice, rs));
-                CK(cudaMemcpyAsync(sf, ck_fy + fld * k, sizeof(A) * fld, cudaMemcpyDeviceToDevice, rs));
-                if (use_graphs && L == C) {
-                    if (!g_rec[set])
-                        capture(rs, &g_rec[set], [&] {
-                            for (int64_t j = 0; j + 1 < C; ++j)
-                                launch_pdl(k_fwd_slot<St>, rs, (const St*)sp + popn * j, sp + popn * (j + 1), sf + fld * j,
-                                                                    sf + fld * (j + 1), G, table, S, sd_rec, j);
-                        });
+                CK(cudaMemcpyAsync(setp[set], ck_pop + popn * k, sizeof(St) * popn, cudaMemcpyDeviceToDevice, rs));
+                CK(cudaMemcpyAsync(setf[set], ck_fy + fld * k, sizeof(A) * fld, cudaMemcpyDeviceToDevice, rs));
+                if (replayed(k)) {
                     k_set_step<<<1, 1, 0, rs>>>(sd_rec, a);
                     check_launch();
                     CK(cudaGraphLaunch(g_rec[set], rs));
                     launches += C - 1;
                 } else {
                     for (int64_t j = 0; j + 1 < L; ++j) {
-                        launch_pdl(k_fwd_slot<St>, rs, (const St*)sp + popn * j, sp + popn * (j + 1), sf + fld * j,
-                                                            sf + fld * (j + 1), G, table, S, nullptr, a + j);
+                        fwd_step(rs, set, j, false, nullptr, a + j);
                         check_launch();
                     }
                 }
@@ -1078,67 +1093,22 @@ struct Impl final : Solver {
             auto sweep = [&](int64_t k) {
                 const int set = int(k & 1);
                 const int64_t a = 1 + k * C, L = seg_len(k);
-                St* sp = setp[set];
-                A* sf = setf[set];
                 CK(cudaStreamWaitEvent(hs, ev_rec[k], 0));
-                if (use_graphs && L == C) {
+                if (replayed(k)) {
                     if (cp != 0) throw ArgError{CAV_ERR_STATE, "adjoint ping-pong out of phase"};
-                    if (!g_adj[set])
-                        capture(stream, &g_adj[set], [&] {
-                            int q = 0;
-                            for (int64_t j = C - 1; j >= 0; --j) {
-                                launch_pdl(k_adj_step<St>, stream, (const St*)sp + popn * j, sf + fld * j, P[q], P[q ^ 1],
-                                                                        acc_cs_d, acc_th_d, G, table, S, sd_adj, j,
-                                                                        obj, j > 0 ? (const St*)sp + popn * (j - 1) : nullptr,
-                                                                        j > 0 ? (const A*)sf + fld * (j - 1) : nullptr);
-                                q ^= 1;
-                            }
-                        });
                     k_set_step<<<1, 1, 0, hs>>>(sd_adj, a);
                     check_launch();
                     CK(cudaGraphLaunch(g_adj[set], hs));
                     launches += C;
                 } else {
                     for (int64_t j = L - 1; j >= 0; --j) {
-                        launch_pdl(k_adj_step<St>, hs, (const St*)sp + popn * j, sf + fld * j, P[cp], P[cp ^ 1],
-                                                                acc_cs_d, acc_th_d, G, table, S, nullptr, a + j, obj,
-                                                                j > 0 ? (const St*)sp + popn * (j - 1) : nullptr,
-                                                                j > 0 ? (const A*)sf + fld * (j - 1) : nullptr);
+                        adj_step(hs, set, j, cp, false, nullptr, a + j);
                         check_launch();
                         cp ^= 1;
                     }
                 }
                 CK(cudaEventRecord(ev_adj[k], hs));
             };
-            // Build the segment graphs now, outside the timed passes (they only
-            // depend on the buffers, not on the state).
-            if (use_graphs && N - 1 >= C) {
-                const int64_t l0 = launches;
-                for (int set = 0; set < 2; ++set) {
-                    St* sp = setp[set];
-                    A* sf = setf[set];
-                    capture(rs, &g_rec[set], [&] {
-                        for (int64_t j = 0; j + 1 < C; ++j)
-                            launch_pdl(k_fwd_slot<St>, rs, (const St*)sp + popn * j, sp + popn * (j + 1), sf + fld * j,
-                                                                sf + fld * (j + 1), G, table, S, sd_rec, j);
-                    });
-                    capture(stream, &g_adj[set], [&] {
-                        int q = 0;
-                        for (int64_t j = C - 1; j >= 0; --j) {
-                            launch_pdl(k_adj_step<St>, stream, (const St*)sp + popn * j, sf + fld * j, P[q], P[q ^ 1],
-                                                                    acc_cs_d, acc_th_d, G, table, S, sd_adj, j, obj,
-                                                                    j > 0 ? (const St*)sp + popn * (j - 1) : nullptr,
-                                                                    j > 0 ? (const A*)sf + fld * (j - 1) : nullptr);
-                            q ^= 1;
-                        }
-                    });
-                    CK(cudaGraphUpload(g_rec[set], rs));
-                    CK(cudaGraphUpload(g_adj[set], stream));
-                }
-                launches = l0;
-                CK(cudaStreamSynchronize(rs));
-                CK(cudaStreamSynchronize(stream));
-            }
             // ---- forward ----
             CK(cudaEventRecord(ev[0], stream));
             nu_accumulate(false);
@@ -1154,11 +1124,28 @@ struct Impl final : Solver {
                 step(stop - time_step);
                 if (next_ck < n_ck && time_step == 1 + next_ck * C) save_ck(next_ck++);
             }
+            CK(cudaEventRecord(ev[1], stream));
+            // The segments' graphs while the forward pass runs (they depend on
+            // nothing it computes): 5 ms of capture and instantiation for 500
+            // steps, of 139 ms for 20 000 steps of 96 x 384.
+            for (int64_t k = n_ck - 1; k >= 0; --k) {
+                const int set = int(k & 1);
+                if (!replayed(k) || g_rec[set]) continue;
+                capture(&g_rec[set], [&] {
+                    for (int64_t j = 0; j + 1 < C; ++j) fwd_step(rs, set, j, true, sd_rec, j);
+                });
+                capture(&g_adj[set], [&] {
+                    int q = 0;
+                    for (int64_t j = C - 1; j >= 0; --j) {
+                        adj_step(rs, set, j, q, true, sd_adj, j);
+                        q ^= 1;
+                    }
+                });
+            }
             double J = 0.0, jc = 0.0;
             int64_t nacc = 0;
             nu_accumulated(&J, &jc, &nacc);
             nu_accumulate(false);
-            CK(cudaEventRecord(ev[1], stream));
             // ---- reverse ----
             // The P ping-pong must sit in P[0] when the first full-segment
             // graph runs: start in P[1] when the (processed first) partial
