@@ -87,7 +87,30 @@ struct LvlIO {
     int n;    // nx * ny (plane stride)
     int hot, cold;
     int node_off;  // offset of this level's nodes in the rounding streams
+    const unsigned char* keep;  // L0: where coarse_to_fine reads REF and the moments
 };
+
+// A level step's collision constants: with the launch once the viscosity ramp has
+// converged (STEADY; the table's row is a load after the step counter's), else
+// from the table.  The step index is only loaded where the rounding needs it.
+// B200, us per coarse step from the table / with the launch: 256 x 1024 FP32 63.1 /
+// 61.2, FP32 / binary16 58.8 / 57.4.  (k_oct_f2c keeps the table: with the
+// constants in the launch 64 x 256 FP32 took 27.8 us instead of 26.1.)
+template <class A>
+struct LvlCoef {
+    const OctScal<A>* tab;
+    int S, lvl;
+    LvlScal<A> steady;
+};
+template <bool STEADY, bool NEED_STEP, class A>
+__device__ __forceinline__ LvlScal<A> coef_of(const LvlCoef<A>& c, const long long* __restrict__ step_dev, int off,
+                                              long long* s_out) {
+    long long s = 0;
+    if (NEED_STEP || !STEADY) s = *step_dev + off;
+    *s_out = s;
+    return STEADY ? c.steady : c.tab[s < c.S ? s : c.S].l[c.lvl];
+}
+
 template <class St>
 struct LvlPair {
     LvlIO<St> b[2];
@@ -496,10 +519,17 @@ __device__ __forceinline__ void split_k(int k, int nx, float inv_nx, int& x, int
 // One (sub-)step of a level: pull + BC + macroscopic (update_macroscopic_guo,
 // src/octree/cavity.rs:252-325) + no-slip (enforce_wall_velocity[_block],
 // :609-656) -> REF; then the level's next collision -> PC.
-template <class St, bool COARSE>
-__global__ void __launch_bounds__(OT) k_oct_step(LvlPair<St> P, const OctScal<typename Fmt<St>::A>* __restrict__ tab,
-                                                 int S, const long long* __restrict__ step_dev, int off, int lvl,
-                                                 uint32_t seed, int phase, float inv_nx, int collide) {
+//
+// MASK: REF and the moments are written only where L.keep is set.  L0's are read
+// by coarse_to_fine (two columns and rows along each block's edge) and by the
+// host, so every coarse step of a call but its last writes them there alone
+// (B200, 256 x 1024: 22 of 41 stores of most nodes; FP32 / binary16 57.4 -> 54.4 us per
+// coarse step, FP64 121 -> 116).  A template, and for L0 alone: the test costs the other
+// steps more than the stores it spares (their masked nodes lie in every warp).
+template <class St, bool COARSE, bool STEADY, bool MASK>
+__global__ void __launch_bounds__(OT) k_oct_step(LvlPair<St> P, LvlCoef<typename Fmt<St>::A> lc,
+                                                 const long long* __restrict__ step_dev, int off, uint32_t seed,
+                                                 int phase, float inv_nx, int collide) {
     pdl_wait();
     using A = typename Fmt<St>::A;
     constexpr bool SH = Fmt<St>::SHIFT;
@@ -509,7 +539,8 @@ __global__ void __launch_bounds__(OT) k_oct_step(LvlPair<St> P, const OctScal<ty
     // the step index and the collision constants first: the stores below
     // may alias them as far as the compiler knows
     long long s;
-    const LvlScal<A> sc = row_of<A>(tab, S, step_dev, off, &s).l[lvl];
+    const LvlScal<A> sc = coef_of<STEADY, Fmt<St>::SR, A>(lc, step_dev, off, &s);
+    const bool keep = !MASK || L.keep[k];
     int x, y;
     split_k(k, L.nx, inv_nx, x, y);
     const bool ghost = !COARSE && (x == 0 || x == L.nx - 1 || y == 0 || y == L.ny - 1);
@@ -530,11 +561,13 @@ __global__ void __launch_bounds__(OT) k_oct_step(LvlPair<St> P, const OctScal<ty
         wall = (L.hot && x == 1) || (L.cold && x == L.nx - 2) || y == 1 || y == L.ny - 2;
     const A fy_prev = L.fy[k];
     const Macro<A, SH> m = macro_node<A, SH>(f, g, fy_prev, wall);
-    store_pops<St>(L.ref_out, L.n, k, f, g, false, 0, 0, 0);
-    L.mac[k] = SH ? m.drho : m.rho;
-    L.mac[L.n + k] = m.ux;
-    L.mac[2 * L.n + k] = m.uy;
-    L.mac[3 * L.n + k] = m.t;
+    if (keep) {
+        store_pops<St>(L.ref_out, L.n, k, f, g, false, 0, 0, 0);
+        L.mac[k] = SH ? m.drho : m.rho;
+        L.mac[L.n + k] = m.ux;
+        L.mac[2 * L.n + k] = m.uy;
+        L.mac[3 * L.n + k] = m.t;
+    }
     if (ghost || !collide) return;
     A fy_new;
     oct_collide<A, SH>(f, g, m, sc, fy_new);
@@ -551,10 +584,10 @@ __global__ void __launch_bounds__(OT) k_oct_step(LvlPair<St> P, const OctScal<ty
 // REF planes, the BGK update, the g PC planes); they exchange u, v, u^2 and
 // T through shared memory at one barrier.  Same bits as k_oct_step.
 constexpr int OCT_FG = 64;
-template <class St>
-__global__ void __launch_bounds__(2 * OCT_FG) k_oct_step_fg(LvlPair<St> P, const OctScal<float>* __restrict__ tab,
-                                                           int S, const long long* __restrict__ step_dev, int off,
-                                                           int lvl, uint32_t seed, int phase, float inv_nx) {
+template <class St, bool STEADY>
+__global__ void __launch_bounds__(2 * OCT_FG) k_oct_step_fg(LvlPair<St> P, LvlCoef<float> lc,
+                                                           const long long* __restrict__ step_dev, int off,
+                                                           uint32_t seed, int phase, float inv_nx) {
     static_assert(Fmt<St>::SHIFT, "the split step runs the shifted formats");
     pdl_wait();
     __shared__ float xu[OCT_FG], xv[OCT_FG], xq[OCT_FG], xt[OCT_FG];
@@ -564,7 +597,7 @@ __global__ void __launch_bounds__(2 * OCT_FG) k_oct_step_fg(LvlPair<St> P, const
     const int k = blockIdx.x * OCT_FG + j;
     const bool act = k < L.n;
     long long s;
-    const LvlScal<float> sc = row_of<float>(tab, S, step_dev, off, &s).l[lvl];
+    const LvlScal<float> sc = coef_of<STEADY, Fmt<St>::SR, float>(lc, step_dev, off, &s);
     int x = 0, y = 0;
     if (act) split_k(k, L.nx, inv_nx, x, y);
     const bool ghost = x == 0 || x == L.nx - 1 || y == 0 || y == L.ny - 1;
@@ -768,7 +801,7 @@ __global__ void __launch_bounds__(OT) k_oct_c2f(LvlPair<StC> C, LvlPair<StF> F,
     const bool act = j < n_ghost;
     const LvlIO<StC> Lc = blockIdx.y == 0 ? C.b[0] : C.b[1];
     const LvlIO<StF> Lf = blockIdx.y == 0 ? F.b[0] : F.b[1];
-    const long long key = (*step_dev + off) * 16 + phase;
+    const long long key = Fmt<StF>::SR ? (*step_dev + off) * 16 + phase : 0;
     A c[NC];
     int kf = 0;
     if (act) {
@@ -1349,6 +1382,7 @@ struct OctImpl final : Octree {
         A* fy = nullptr;
         int hot = 0, cold = 0, node_off = 0;
         int cur = 0;  // REF and PC buffers flip together
+        unsigned char* keep = nullptr;
         LvlIO<St> io() const {
             LvlIO<St> o;
             o.ref_in = ref[cur];
@@ -1363,6 +1397,7 @@ struct OctImpl final : Octree {
             o.hot = hot;
             o.cold = cold;
             o.node_off = node_off;
+            o.keep = keep;
             return o;
         }
         // The current state: REF and PC written by the last step (the
@@ -1394,7 +1429,10 @@ struct OctImpl final : Octree {
     uint32_t seed32 = 0;
     bool pc_valid = false;
     Xi<A> xa{}, xb{};
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};
+    // OCT_GRAPH_STEPS coarse steps: [steady scalars][the call's last][L0 buffer]
+    cudaGraphExec_t graph[2][2][2] = {};
+    bool steady_now = false;  // the launches being made are past the viscosity ramp
+    OctScal<A> steady_row{};
     int level_kernel = CAV_OCT_LEVEL_FG;  // fine-level step form (step_fine)
     // dynamic mixed-scale SGS model (set_dynamic_sgs, src/octree/solver.rs:476-481)
     bool dyn = false;
@@ -1413,12 +1451,21 @@ struct OctImpl final : Octree {
     std::vector<void*> allocs;
 
     ~OctImpl() override {
-        for (auto& gx : graph)
-            if (gx) cudaGraphExecDestroy(gx);
+        drop_graphs();
         for (auto& gx : dgraph)
             if (gx) cudaGraphExecDestroy(gx);
         for (void* b : allocs) cudaFree(b);
         if (stream) cudaStreamDestroy(stream);
+    }
+
+    void drop_graphs() {
+        for (auto& a : graph)
+            for (auto& b : a)
+                for (auto& gx : b)
+                    if (gx) {
+                        cudaGraphExecDestroy(gx);
+                        gx = nullptr;
+                    }
     }
 
     template <class T>
@@ -1617,6 +1664,15 @@ struct OctImpl final : Octree {
             upload_coin(g2, co2, n_co2_0, n_co2_1);
         }
 
+        // L0's nodes that coarse_to_fine reads
+        std::vector<unsigned char> keep(size_t(L0.n), 0);
+        for (const HostGrid& g : g1)
+            for (const auto& e : g.ghosts)
+                for (int k : e.kc) keep[k] = 1;
+        L0.keep = dalloc<unsigned char>(keep.size());
+        CK(cudaMemcpyAsync(L0.keep, keep.data(), keep.size(), cudaMemcpyHostToDevice, stream));
+        CK(cudaStreamSynchronize(stream));
+
         // per-step table: rows until the ramps have converged bit for bit
         std::vector<OctScal<A>> rows;
         rows.push_back(row(0));
@@ -1629,6 +1685,7 @@ struct OctImpl final : Octree {
             }
         }
         S = int(rows.size()) - 1;
+        steady_row = rows.back();
         tab = dalloc<OctScal<A>>(rows.size());
         CK(cudaMemcpyAsync(tab, rows.data(), sizeof(OctScal<A>) * rows.size(), cudaMemcpyHostToDevice, stream));
         step_dev = dalloc<long long>(1);
@@ -1847,6 +1904,7 @@ struct OctImpl final : Octree {
         launch(k_oct_c2f<StF, StF>, grid_of(4 * n_ghost2, 2), c, f, (const GhostE<A>*)gh2, n_ghost2, xb, xi_b_dev(),
                (const long long*)step_dev, j, seed32, 4);
     }
+    LvlCoef<A> coef(int lvl) const { return LvlCoef<A>{tab, S, lvl, steady_row.l[lvl]}; }
     void f2c_L2(int off) {
         LvlPair<StF> f = pair_cur(L2[0], L2[1]);
         LvlPair<StF> c = pair_cur(L1[0], L1[1]);
@@ -1860,10 +1918,12 @@ struct OctImpl final : Octree {
         launch(k_oct_f2c<StF, StC>, f2c_grid(std::max(n_co0, n_co1)), f, c, (const CoinE*)co1, n_co0, n_co1,
                xa, xi_a_dev(), (const OctScal<A>*)tab, S, (const long long*)step_dev, off, 0, seed32, 13, int(!dyn));
     }
-    void step_L0(int j) {
+    void step_L0(int j, bool mask) {
         LvlPair<StC> q = pair(L0, L0);
-        launch(k_oct_step<StC, true>, grid_of(L0.n, 1), q, (const OctScal<A>*)tab, S, (const long long*)step_dev, j + 1,
-               0, seed32, 1, 1.0f / float(L0.nx), int(!dyn));
+        launch(steady_now ? (mask ? k_oct_step<StC, true, true, true> : k_oct_step<StC, true, true, false>)
+                          : (mask ? k_oct_step<StC, true, false, true> : k_oct_step<StC, true, false, false>),
+               grid_of(L0.n, 1), q, coef(0), (const long long*)step_dev, j + 1, seed32, 1, 1.0f / float(L0.nx),
+               int(!dyn));
         L0.cur ^= 1;
     }
     // A fine level's (sub-)step: the f and g halves of a node on two threads
@@ -1872,19 +1932,19 @@ struct OctImpl final : Octree {
     bool split_fg() const { return level_kernel == CAV_OCT_LEVEL_FG && Fmt<StF>::SHIFT && !dyn && p.cs == 0.0; }
     void step_fine(Lvl<StF>* Lv, int lvl, int off, int phase) {
         LvlPair<StF> q = pair(Lv[0], Lv[1]);
+        const float inv_nx = 1.0f / float(Lv[0].nx);
+        Lv[0].cur ^= 1;
+        Lv[1].cur ^= 1;
         if constexpr (Fmt<StF>::SHIFT) {
             if (split_fg()) {
-                launch(k_oct_step_fg<StF>, dim3((Lv[0].n + OCT_FG - 1) / OCT_FG, 2), q, (const OctScal<float>*)tab, S,
-                       (const long long*)step_dev, off, lvl, seed32, phase, 1.0f / float(Lv[0].nx));
-                Lv[0].cur ^= 1;
-                Lv[1].cur ^= 1;
+                launch(steady_now ? k_oct_step_fg<StF, true> : k_oct_step_fg<StF, false>,
+                       dim3((Lv[0].n + OCT_FG - 1) / OCT_FG, 2), q, coef(lvl), (const long long*)step_dev, off, seed32,
+                       phase, inv_nx);
                 return;
             }
         }
-        launch(k_oct_step<StF, false>, grid_of(Lv[0].n, 2), q, (const OctScal<A>*)tab, S, (const long long*)step_dev,
-               off, lvl, seed32, phase, 1.0f / float(Lv[0].nx), int(!dyn));
-        Lv[0].cur ^= 1;
-        Lv[1].cur ^= 1;
+        launch(steady_now ? k_oct_step<StF, false, true, false> : k_oct_step<StF, false, false, false>,
+               grid_of(Lv[0].n, 2), q, coef(lvl), (const long long*)step_dev, off, seed32, phase, inv_nx, int(!dyn));
     }
     void step_L1(int off, int phase) { step_fine(L1, 1, off, phase); }
     void step_L2(int off, int phase) { step_fine(L2, 2, off, phase); }
@@ -1894,12 +1954,12 @@ struct OctImpl final : Octree {
             throw ArgError{CAV_ERR_ARG, "unknown octree level kernel"};
         if (kind == level_kernel) return;
         CK(cudaStreamSynchronize(stream));
-        for (auto* gs : {graph, dgraph})
-            for (int i = 0; i < 2; ++i)
-                if (gs[i]) {
-                    CK(cudaGraphExecDestroy(gs[i]));
-                    gs[i] = nullptr;
-                }
+        drop_graphs();
+        for (auto& gx : dgraph)
+            if (gx) {
+                CK(cudaGraphExecDestroy(gx));
+                gx = nullptr;
+            }
         level_kernel = kind;
     }
     int get_level_kernel() const override { return level_kernel; }
@@ -1941,11 +2001,7 @@ struct OctImpl final : Octree {
         // its graphs are captured anew with the device factors
         if (dyn && !on) {
             pc_valid = false;
-            for (auto& gx : graph)
-                if (gx) {
-                    CK(cudaGraphExecDestroy(gx));
-                    gx = nullptr;
-                }
+            drop_graphs();
         }
         dyn = on;
         dyn_alpha = smag_alpha;
@@ -2034,7 +2090,7 @@ struct OctImpl final : Octree {
             launch_b(k_oct_mean_parts<A>, dim3(DYN_PARTS, 3), dim3(256), J, mpart);
             launch_b(k_oct_xi<A>, dim3(1), dim3(32), J, (const double*)mpart, xi_dev, dstat + 5);
         }
-        step_L0(j);
+        step_L0(j, false);
         c2f_L1(j);
         const double tau_mol_l1 = 0.5 + 3.0 * 2.0 * nu_eff, tau_mol_l2 = 0.5 + 3.0 * 4.0 * nu_eff;
         sgs_levels<false>(L1, 2, nut1, tau_mol_l1, 2.0 * nu_eff, 2.0 * al_eff, j, 1, 3);
@@ -2130,8 +2186,9 @@ struct OctImpl final : Octree {
 
     // One step_cavity (src/octree/solver.rs:647-947), all launches on `stream`,
     // with the step index *step_dev + j.
-    void launch_coarse_step(int j) {
-        step_L0(j);
+    // last: the call's last coarse step, whose REF state the host may read.
+    void launch_coarse_step(int j, bool last) {
+        step_L0(j, !last);
         c2f_L1(j);
         step_L1(j, 3);
         if (levels == 3) {
@@ -2148,13 +2205,13 @@ struct OctImpl final : Octree {
         launch_b(k_add_step, dim3(1), dim3(1), step_dev, (long long)n);
     }
 
-    cudaGraphExec_t get_graph() {
-        cudaGraphExec_t& gx = graph[L0.cur];
+    cudaGraphExec_t get_graph(bool last) {
+        cudaGraphExec_t& gx = graph[steady_now][last][L0.cur];
         if (gx) return gx;
         const int c0 = L0.cur, c1 = L1[0].cur, c2 = L2[0].cur;
         const int64_t l0 = launches;
         CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        for (int j = 0; j < OCT_GRAPH_STEPS; ++j) launch_coarse_step(j);
+        for (int j = 0; j < OCT_GRAPH_STEPS; ++j) launch_coarse_step(j, last && j + 1 == OCT_GRAPH_STEPS);
         add_steps(OCT_GRAPH_STEPS);
         cudaGraph_t gr;
         CK(cudaStreamEndCapture(stream, &gr));
@@ -2220,18 +2277,19 @@ struct OctImpl final : Octree {
         if (!pc_valid) collide_all();
         set_step_dev();
         while (n > 0) {
+            steady_now = time_step >= S;
             if (n >= OCT_GRAPH_STEPS) {
-                cudaGraphExec_t gx = get_graph();
-                CK(cudaGraphLaunch(gx, stream));
+                CK(cudaGraphLaunch(get_graph(n == OCT_GRAPH_STEPS), stream));
                 launches += int64_t(OCT_GRAPH_STEPS) * per_step_launches() + 1;
                 time_step += OCT_GRAPH_STEPS;
                 n -= OCT_GRAPH_STEPS;
             } else {
-                launch_coarse_step(0);
+                launch_coarse_step(0, n == 1);
                 add_steps(1);
                 time_step += 1;
                 n -= 1;
             }
+            steady_now = false;
             step_dev_val = time_step;
         }
         CK(cudaGetLastError());
