@@ -37,7 +37,25 @@ struct BatchItem {
     int cav, tx0, ty0, rows;
 };
 
+// A work item with its cavity beside it, for the one-CTA-per-item kernels: a CTA
+// reads it and its scalars' row, and nothing else stands before its population
+// loads (with the cavity looked up by the item's index, and the row by the
+// cavity's spin-up, three loads in a row did: B200, 64 cavities, us per step f16sr
+// 40.0 / 38.9
+// and FP32 48.1 / 45.7 with k_batch_x, bfloat16 37.3 / 36.1, its stochastic form 39.8 /
+// 41.0).
+template <class St>
+struct BatchWork {
+    BatchCav<St> cv;
+    BatchItem item;
+};
+
 constexpr int BATCH_THREADS = 128;
+
+// The scalar table's row of step s: row r holds every cavity's scalars of step
+// min(r, its spin-up), the last one (n_rows - 1 = the longest spin-up) the
+// steady state of all.
+__device__ __forceinline__ long long scalar_row(long long s, int n_rows) { return s < n_rows - 1 ? s : n_rows - 1; }
 // Largest state of the cavities stepped together (Batch::setup_groups).  The
 // 64-cavity sweep (2.29 M nodes: 340 MB in FP32, 175 MB in 16 bits) on a B200,
 // us per lattice step against the groups' size in MB:
@@ -80,27 +98,27 @@ __global__ void __launch_bounds__(BATCH_THREADS)
 // are not kept live across items, so the kernel needs the registers of
 // k_fused, not of k_batch; capped at 56 (with 128-thread CTAs, 9 resident
 // per SM; a word or three spilled to L1; on a B200 +3 % binary16, +15 %
-// bfloat16 with stochastic rounding against 64 registers and 8 CTAs).
+// bfloat16 with stochastic rounding against 64 registers and 8 CTAs).  FP64's
+// node needs 156 and spills at 56: 128 there (64 cavities: 370 -> 145 us).
 template <class St, bool WRITE_NUT>
-__global__ void __maxnreg__(56)
-    k_batch_np(const BatchCav<St>* __restrict__ cavs, const BatchItem* __restrict__ items,
-               const StepScalars<typename Fmt<St>::A>* __restrict__ table, int n_cav, long long step,
-               const long long* __restrict__ step_dev) {
+__global__ void __maxnreg__((std::is_same<St, double>::value ? 128 : 56))
+    k_batch_np(const BatchWork<St>* __restrict__ work, const StepScalars<typename Fmt<St>::A>* __restrict__ table,
+               int n_rows, int n_cav, long long step, const long long* __restrict__ step_dev) {
     using A = typename Fmt<St>::A;
     pdl_wait();
     const long long s = step_dev ? *step_dev + step : step;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const BatchItem item = items[blockIdx.x];
-    const BatchCav<St>& cv = cavs[item.cav];
-    const int row = s < cv.spin_up ? int(s) : cv.spin_up;
-    StepScalars<A> c = table[(long long)row * n_cav + item.cav];
+    const BatchWork<St>& wk = work[blockIdx.x];
+    const BatchItem item = wk.item;
+    StepScalars<A> c = table[scalar_row(s, n_rows) * n_cav + item.cav];
     c.step = s;
     c.step_dev = nullptr;
-    const int cur = (cv.parity + int(s & 1)) & 1;
+    St *const p0 = wk.cv.pop[0], *const p1 = wk.cv.pop[1];
+    const bool cur = (wk.cv.parity + int(s & 1)) & 1;
     const int ix = item.tx0 + lane;
-    if (ix < cv.G.nx && w < item.rows)
-        fused_node<St, WRITE_NUT, false, false>(cv.pop[cur], cv.pop[cur ^ 1], cv.fy, cv.nut, nullptr, nullptr, cv.G,
-                                                ix, item.ty0 + w, c);
+    if (ix < wk.cv.G.nx && w < item.rows)
+        fused_node<St, WRITE_NUT, false, false>(cur ? p1 : p0, cur ? p0 : p1, wk.cv.fy, wk.cv.nut, nullptr, nullptr,
+                                                wk.cv.G, ix, item.ty0 + w, c);
 }
 
 // k_batch_np with two rows per thread (fused_pair: the arithmetic of both
@@ -110,23 +128,22 @@ __global__ void __maxnreg__(56)
 // spill traffic on a B200.
 template <class St, bool WRITE_NUT>
 __global__ void __maxnreg__(96)
-    k_batch_np2(const BatchCav<St>* __restrict__ cavs, const BatchItem* __restrict__ items,
-                const StepScalars<float>* __restrict__ table, int n_cav, long long step,
-                const long long* __restrict__ step_dev) {
+    k_batch_np2(const BatchWork<St>* __restrict__ work, const StepScalars<float>* __restrict__ table, int n_rows,
+                int n_cav, long long step, const long long* __restrict__ step_dev) {
     pdl_wait();
     const long long s = step_dev ? *step_dev + step : step;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const BatchItem item = items[blockIdx.x];
-    const BatchCav<St>& cv = cavs[item.cav];
-    const int row = s < cv.spin_up ? int(s) : cv.spin_up;
-    StepScalars<float> c = table[(long long)row * n_cav + item.cav];
+    const BatchWork<St>& wk = work[blockIdx.x];
+    const BatchItem item = wk.item;
+    StepScalars<float> c = table[scalar_row(s, n_rows) * n_cav + item.cav];
     c.step = s;
     c.step_dev = nullptr;
-    const int cur = (cv.parity + int(s & 1)) & 1;
+    St *const p0 = wk.cv.pop[0], *const p1 = wk.cv.pop[1];
+    const bool cur = (wk.cv.parity + int(s & 1)) & 1;
     const int ix = item.tx0 + lane;
-    if (ix < cv.G.nx && 2 * w < item.rows)
-        fused_pair<St, WRITE_NUT, false>(cv.pop[cur], cv.pop[cur ^ 1], cv.fy, cv.nut, nullptr, nullptr, cv.G, ix,
-                                         item.ty0 + 2 * w, 2 * w + 1 < item.rows, c);
+    if (ix < wk.cv.G.nx && 2 * w < item.rows)
+        fused_pair<St, WRITE_NUT, false>(cur ? p1 : p0, cur ? p0 : p1, wk.cv.fy, wk.cv.nut, nullptr, nullptr, wk.cv.G,
+                                         ix, item.ty0 + 2 * w, 2 * w + 1 < item.rows, c);
 }
 
 // The node-pair body of k_fused_x (xpair.cuh: two x-adjacent nodes per
@@ -134,23 +151,22 @@ __global__ void __maxnreg__(96)
 // 64-column x rows) item: warp w takes row ty0 + w.
 template <class St, bool WRITE_NUT>
 __global__ void __maxnreg__(XPAIR_MAXNREG)
-    k_batch_x(const BatchCav<St>* __restrict__ cavs, const BatchItem* __restrict__ items,
-              const StepScalars<float>* __restrict__ table, int n_cav, long long step,
-              const long long* __restrict__ step_dev) {
+    k_batch_x(const BatchWork<St>* __restrict__ work, const StepScalars<float>* __restrict__ table, int n_rows,
+              int n_cav, long long step, const long long* __restrict__ step_dev) {
     pdl_wait();
     const long long s = step_dev ? *step_dev + step : step;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const BatchItem item = items[blockIdx.x];
-    const BatchCav<St>& cv = cavs[item.cav];
-    const int row = s < cv.spin_up ? int(s) : cv.spin_up;
-    StepScalars<float> c = table[(long long)row * n_cav + item.cav];
+    const BatchWork<St>& wk = work[blockIdx.x];
+    const BatchItem item = wk.item;
+    StepScalars<float> c = table[scalar_row(s, n_rows) * n_cav + item.cav];
     c.step = s;
     c.step_dev = nullptr;
-    const int cur = (cv.parity + int(s & 1)) & 1;
+    St *const p0 = wk.cv.pop[0], *const p1 = wk.cv.pop[1];
+    const bool cur = (wk.cv.parity + int(s & 1)) & 1;
     const int ix = item.tx0 + 2 * lane;
-    if (ix < cv.G.nx && w < item.rows)
-        fused_xpair<St, WRITE_NUT, false>(cv.pop[cur], cv.pop[cur ^ 1], cv.fy, cv.fy, cv.nut, nullptr, nullptr, cv.G,
-                                          ix, item.ty0 + w, c);
+    if (ix < wk.cv.G.nx && w < item.rows)
+        fused_xpair<St, WRITE_NUT, false>(cur ? p1 : p0, cur ? p0 : p1, wk.cv.fy, wk.cv.fy, wk.cv.nut, nullptr, nullptr,
+                                          wk.cv.G, ix, item.ty0 + w, c);
 }
 
 // Which kernel runs a batched step, and the parameters it uses:
@@ -199,6 +215,10 @@ struct Batch final : BatchBase {
     std::vector<Impl<St>*> cv;
     BatchCav<St>* d_cavs = nullptr;
     BatchItem* d_items = nullptr;
+    BatchWork<St>* d_work = nullptr;  // the items of kernels 3, 4 and 5 with their cavities
+    std::vector<BatchItem> items;     // the current kernel's work list
+    std::vector<BatchCav<St>> hcavs;  // host copy of d_cavs
+    bool work_dirty = true;
     StepScalars<A>* d_table = nullptr;
     long long* step_dev = nullptr;
     long long step_dev_val = -1;
@@ -231,7 +251,7 @@ struct Batch final : BatchBase {
         for (Group& g : groups)
             if (g.graph) cudaGraphExecDestroy(g.graph);
         if (h_err) cudaFreeHost(h_err);
-        void* bufs[] = {d_cavs,      d_items,     d_table, step_dev, d_tcavs,   d_maps[1],
+        void* bufs[] = {d_cavs,      d_items, d_work,     d_table, step_dev, d_tcavs,   d_maps[1],
                         d_maps[2],   d_titems[1], d_titems[2], d_err,  d_xmaps[0],
                         d_xmaps[1],  d_xitems[0], d_xitems[1], d_fmaps[0], d_fmaps[1]};
         for (void* b : bufs)
@@ -405,7 +425,7 @@ struct Batch final : BatchBase {
         tun = t;
         // work items: 64 columns for the node-pair kernel, 32 otherwise
         const int width = k == 5 ? 64 : 32;
-        std::vector<BatchItem> items;
+        items.clear();
         for (int i = 0; i < int(cv.size()); ++i) {
             const int nx = cv[i]->p.nx, ny = cv[i]->p.ny;
             for (int y0 = 0; y0 < ny; y0 += r)
@@ -430,6 +450,7 @@ struct Batch final : BatchBase {
             g.item0 = first[g.c0];
             g.n_items = first[g.c1] - first[g.c0];
         }
+        work_dirty = true;
         drop_graphs();
         CK(cudaStreamSynchronize(stream));
     }
@@ -462,7 +483,8 @@ struct Batch final : BatchBase {
         for (auto* c : cv)
             if (c->time_step != time_step) throw ArgError{CAV_ERR_STATE, "cavities of a batch out of step"};
         if (cavs_dirty) {
-            std::vector<BatchCav<St>> h(cv.size());
+            std::vector<BatchCav<St>>& h = hcavs;
+            h.resize(cv.size());
             for (size_t i = 0; i < cv.size(); ++i) {
                 auto* c = cv[i];
                 h[i].pop[0] = c->pop[0];
@@ -489,6 +511,19 @@ struct Batch final : BatchBase {
             CK(cudaMemcpyAsync(d_tcavs, t.data(), sizeof(TileCav<St>) * t.size(), cudaMemcpyHostToDevice, stream));
             CK(cudaStreamSynchronize(stream));
             cavs_dirty = false;
+            work_dirty = true;
+        }
+        const int k = effective_kernel(tun.kernel);
+        if (work_dirty && k >= 3 && k <= 5) {
+            std::vector<BatchWork<St>> w(items.size());
+            for (size_t i = 0; i < items.size(); ++i) w[i] = BatchWork<St>{hcavs[items[i].cav], items[i]};
+            if (d_work) CK(cudaFree(d_work));
+            d_work = nullptr;
+            drop_graphs();
+            CK(cudaMalloc(&d_work, sizeof(BatchWork<St>) * w.size()));
+            CK(cudaMemcpyAsync(d_work, w.data(), sizeof(BatchWork<St>) * w.size(), cudaMemcpyHostToDevice, stream));
+            CK(cudaStreamSynchronize(stream));
+            work_dirty = false;
         }
     }
 
@@ -513,7 +548,7 @@ struct Batch final : BatchBase {
     // The one-CTA-per-item kernels (3, 4, 5) over d_items.
     template <bool WN>
     void launch_np(const Group& g, int k, const long long* sdev, long long step) {
-        const BatchItem* const items = d_items + g.item0;
+        const BatchWork<St>* const work = d_work + g.item0;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(g.n_items);
         cfg.blockDim = dim3(32 * tun.rows_per_item);
@@ -526,21 +561,21 @@ struct Batch final : BatchBase {
         cfg.numAttrs = 1;
         if constexpr (has_pairs<St>::value) {
             if (k == 5) {
-                CK(cudaLaunchKernelEx(&cfg, k_batch_x<St, WN>, (const BatchCav<St>*)d_cavs, items,
-                                      (const StepScalars<float>*)d_table, int(cv.size()), step, sdev));
+                CK(cudaLaunchKernelEx(&cfg, k_batch_x<St, WN>, work, (const StepScalars<float>*)d_table, table_rows,
+                                      int(cv.size()), step, sdev));
                 return;
             }
         }
         if constexpr (Fmt<St>::SHIFT) {
             if (k == 4) {
                 cfg.blockDim = dim3(16 * tun.rows_per_item);
-                CK(cudaLaunchKernelEx(&cfg, k_batch_np2<St, WN>, (const BatchCav<St>*)d_cavs,
-                                      items, (const StepScalars<float>*)d_table, int(cv.size()), step, sdev));
+                CK(cudaLaunchKernelEx(&cfg, k_batch_np2<St, WN>, work, (const StepScalars<float>*)d_table, table_rows,
+                                      int(cv.size()), step, sdev));
                 return;
             }
         }
-        CK(cudaLaunchKernelEx(&cfg, k_batch_np<St, WN>, (const BatchCav<St>*)d_cavs, items,
-                              (const StepScalars<A>*)d_table, int(cv.size()), step, sdev));
+        CK(cudaLaunchKernelEx(&cfg, k_batch_np<St, WN>, work, (const StepScalars<A>*)d_table, table_rows,
+                              int(cv.size()), step, sdev));
     }
 
     template <int TY, bool WN>
