@@ -41,9 +41,8 @@ struct BatchItem {
 // reads it and its scalars' row, and nothing else stands before its population
 // loads (with the cavity looked up by the item's index, and the row by the
 // cavity's spin-up, three loads in a row did: B200, 64 cavities, us per step f16sr
-// 40.0 / 38.9
-// and FP32 48.1 / 45.7 with k_batch_x, bfloat16 37.3 / 36.1, its stochastic form 39.8 /
-// 41.0).
+// 40.0 / 38.9 and FP32 48.1 / 45.7 with k_batch_x, bfloat16 37.3 / 36.1, its
+// stochastic form 39.8 / 41.0).
 template <class St>
 struct BatchWork {
     BatchCav<St> cv;

@@ -164,22 +164,31 @@ struct Impl final : Solver {
     // Block height of the one-node kernels: 32 x 4 for FP32 storage, 32 x 2
     // otherwise (a B200 takes about 1 us to start 1000 CTAs, so FP32's short
     // steps want few; FP64's 156 registers leave 32 x 4 a coarser fit: 64 x 256
-    // 2.59 us against 2.54).
+    // 2.18 us against 2.16), except for a handful of CTAs, where fewer share more
+    // of the instruction stream and the L2 (16 x 40: 1.83 against 2.04; 32 x 64, 16
+    // CTAs: 2.03 against 2.06; level from 24 x 96 on).
     static constexpr int BYF = std::is_same<St, float>::value ? 4 : BY;
+    static constexpr int F64_FEW_CTAS = 16;
     dim3 blk{BX, BYF}, grd{};
     // the node-pair kernel: 32 x BYX threads cover 64 columns x BYX rows
     static constexpr int BYX = X_ROWS;
     dim3 blkx{BX, BYX}, grdx{};
-    // the 16-bit formats' default step kernel: pairs split over two warps
-    // for cavities that cannot fill the GPU (a step is then one thread's
-    // latency chain; on a B200 128 x 512 f16sr 2.25 us against 2.35, 64 x 256
-    // 1.74 against 2.00), plain pairs above (256 x 768: 4.2 against 5.1)
+    // the 16-bit formats' default step kernel: pairs split over two warps for
+    // cavities that cannot fill the GPU (a step is then one thread's latency
+    // chain; on a B200 96 x 384 f16sr 2.10 us against 2.15, 180 x 380 2.38 against
+    // 2.44, 128 x 512 level), as long as every CTA runs at once: 4 of 128 threads
+    // fit on an SM, and what is left over costs a second wave (130 x 500, 750 CTAs:
+    // 3.40 against 2.67 with plain pairs; 4 x 2000, 1000 CTAs: 3.79 against 2.96).
+    // The node limit is where plain pairs catch up in a full wave (192 x 388:
+    // 2.31 against 2.28; f16g, whose g half is the longer, 128 x 590: 3.01 against 2.90)
+    static constexpr int SPLIT_CTAS = 4;
     static constexpr long long SPLIT_MAX_NODES = 70000;
     int kern = is_p16<St>::value ? 1 : 0;
     // FP32 (step kernel 0): one node per thread while one thread's chain is
     // all there is (96 x 384 1.80 us per step against 1.96 for split pairs),
     // pairs split over two warps once issue counts too (128 x 512: 2.19 against
-    // 2.40), plain pairs above (512 x 1024: 8.8 against 9.2 and 11.6).
+    // 2.40) and they run at once, plain pairs above (130 x 530: 2.59 against 3.21;
+    // 512 x 1024: 8.8 against 9.2, one node per thread 11.6).
     static constexpr long long F32_NODE_MAX = 48000;
     int f32_form = 1;
     // FP64: k_fused at 128 registers (8 CTAs of 64 threads per SM, a few
@@ -216,13 +225,17 @@ struct Impl final : Solver {
         G.plane = (long long)p.ny * pitch;
         if ((long long)NPLANES * G.plane >= (1ll << 31))
             throw ArgError{CAV_ERR_ARG, "grid too large: 18 * ny * pitch must stay below 2^31 elements"};
-        grd = dim3((p.nx + BX - 1) / BX, (p.ny + BYF - 1) / BYF);
+        const int nbx = (p.nx + BX - 1) / BX;
+        if (std::is_same<St, double>::value && nbx * ((p.ny + 3) / 4) <= F64_FEW_CTAS) blk.y = 4;
+        grd = dim3(nbx, (p.ny + blk.y - 1) / blk.y);
         grdx = dim3(((p.nx + 1) / 2 + BX - 1) / BX, (p.ny + BYX - 1) / BYX);
-        if (is_p16<St>::value && (long long)p.nx * p.ny <= SPLIT_MAX_NODES) kern = 2;
-        const long long nodes = (long long)p.nx * p.ny;
-        f32_form = nodes <= F32_NODE_MAX ? 0 : (nodes <= SPLIT_MAX_NODES ? 2 : 1);
         int n_sm = 0;
         CK(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, p.device));
+        const long long split_ctas = (long long)grdx.x * ((p.ny + XS_ROWS - 1) / XS_ROWS);
+        const long long nodes = (long long)p.nx * p.ny;
+        const int pairs = split_ctas <= (long long)SPLIT_CTAS * n_sm && nodes <= SPLIT_MAX_NODES ? 2 : 1;
+        if (is_p16<St>::value) kern = pairs;
+        f32_form = nodes <= F32_NODE_MAX ? 0 : pairs;
         f64_packed = (long long)grd.x * grd.y > (long long)F64_CTAS * n_sm;
         if (!stream) {
             CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));

@@ -198,8 +198,10 @@ int cav_launch_count(cav_handle* h, int64_t* n);
  * CAV_STEP_PAIR_SPLIT the same node pairs with the f and g halves of each
  * pair's work on two warps (twice the warps, each a shorter chain: for
  * cavities too small to fill the GPU).  Default for the 16-bit formats:
- * CAV_STEP_PAIR_SPLIT up to 70 000 nodes, CAV_STEP_PAIR above; FP64 / FP32:
- * CAV_STEP_NODE.  All give the same bits; CAV_ERR_ARG for a pair kernel on
+ * CAV_STEP_PAIR_SPLIT up to 70 000 nodes while all its blocks of 64 x 2 nodes
+ * run at once (four per SM), CAV_STEP_PAIR otherwise; FP64 / FP32:
+ * CAV_STEP_NODE, with which FP32 takes the library's own choice among the same
+ * three by size.  All give the same bits; CAV_ERR_ARG for a pair kernel on
  * FP64 / FP32. */
 #define CAV_STEP_NODE 0
 #define CAV_STEP_PAIR 1
