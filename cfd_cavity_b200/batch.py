@@ -1,5 +1,6 @@
 """Python mirror of the batch C ABI (``cav_batch_*``): many cavities advanced
-in lockstep by one kernel launch per lattice step.
+together, one kernel launch per lattice step and per group of cavities whose
+state fits the L2.
 
 The reference runs one cavity per process (``src/main.rs:42-443``); a batch
 is a set of ``CavitySolver::new`` objects stepped together.  Each cavity of a
@@ -150,7 +151,7 @@ class CavityBatch:
         node per thread (1, 2, 4 or 8 rows); 4: the same items, two rows per
         thread on packed FP32x2 arithmetic (2, 4 or 8 rows); 5: one CTA per
         64-column x rows_per_item item, two x-adjacent nodes per thread
-        (16-bit formats; 1, 2, 4 or 8 rows); 6: the node-pair body on
+        (16-bit formats and FP32; 1, 2, 4 or 8 rows); 6: the node-pair body on
         TMA-staged tiles of 64 columns x rows_per_item rows (4 or 8),
         ctas_per_sm persistent CTAs per SM (16-bit formats)."""
         t = L.CavBatchTuning(rows_per_item, ctas_per_sm, int(kernel))

@@ -234,8 +234,10 @@ int cav_restart_from_snapshot(cav_handle* h, const char* path);
  * alpha_t per node before every collision with the dynamic mixed-scale model
  * (compute_dynamic_sgs, :562-828) instead of Cs^2 |S| and nu_t / Pr_t.
  * Reference defaults: smag_alpha 0.5, nu_sm_min -0.1, eta_test 2.0
- * (src/cli.rs:118-120).  A step then runs the model's four kernels, the
- * collision and the streaming as separate launches (no graph replay). */
+ * (src/cli.rs:118-120).  A step with the default eta_test then runs as three
+ * launches: the strains and test-filter contractions, the coefficients with
+ * the collision, and the streaming (five launches for other test widths);
+ * graphs of 16 steps once the viscosity ramp is over. */
 int cav_set_dynamic_sgs(cav_handle* h, int32_t on, double smag_alpha, double nu_sm_min, double eta_test);
 /* out4 = cs_dyn_mean, cs_dyn_max, kappa_dyn_mean, kappa_dyn_max of the last
  * evaluation (the driver's progress line, src/main.rs:181-182); zeros before
@@ -284,8 +286,8 @@ typedef struct cav_batch cav_batch;
  *   4  the same items, two rows per thread on packed FP32x2 arithmetic
  *      (2, 4 or 8 rows; FP64 runs it as 3);
  *   5  one CTA per 64-column x rows_per_item item (1, 2, 4 or 8 rows), two
- *      x-adjacent nodes per thread, each plane one 32-bit word (16-bit
- *      formats; FP64 and FP32 run it as 3);
+ *      x-adjacent nodes per thread, each plane one word (16-bit formats and
+ *      FP32; FP64 runs it as 3);
  *   6  the same node-pair body on TMA-staged shared-memory tiles of 64
  *      columns x rows_per_item rows (4 or 8), ctas_per_sm persistent CTAs per
  *      SM (16-bit formats; FP64 and FP32 run it as 3).
@@ -298,7 +300,9 @@ typedef struct cav_batch_tuning {
 int cav_batch_create(const cav_params* params, int32_t n, cav_batch** out);
 int cav_batch_destroy(cav_batch* b);
 const char* cav_batch_last_error(const cav_batch* b);
-/* n lockstep steps of every cavity (one kernel launch per step). */
+/* n steps of every cavity.  Cavities are independent, so a batch whose state
+ * is larger than the L2 advances group by group, each group fitting it and
+ * taking all n steps before the next (one kernel launch per group and step). */
 int cav_batch_step(cav_batch* b, int64_t n);
 int cav_batch_get_fields(cav_batch* b, int32_t i, double* rho, double* ux, double* uy, double* t,
                          double* nu_t, double* fy);
