@@ -184,11 +184,15 @@ struct Impl final : Solver {
     static constexpr int SPLIT_CTAS = 4;
     static constexpr long long SPLIT_MAX_NODES = 70000;
     int kern = is_p16<St>::value ? 1 : 0;
-    // FP32 (step kernel 0): one node per thread while one thread's chain is
-    // all there is (96 x 384 1.80 us per step against 1.96 for split pairs),
-    // pairs split over two warps once issue counts too (128 x 512: 2.19 against
-    // 2.40) and they run at once, plain pairs above (130 x 530: 2.59 against 3.21;
-    // 512 x 1024: 8.8 against 9.2, one node per thread 11.6).
+    // FP32 (step kernel 0): one node per thread while three CTAs per SM hold the
+    // grid (one thread's chain is all there is: 96 x 384 1.80 us per step against
+    // 1.96 for split pairs; 126 x 386 2.18 against 2.28), pairs split over two
+    // warps while those run at once (128 x 512 2.19 against 2.40, 98 x 470 2.19
+    // against 2.36), and past that plain pairs (130 x 530: 2.59 against 3.21 split;
+    // 512 x 1024: 8.8 against 9.2, one node per thread 11.6) unless the grid is
+    // narrow, where they leave most lanes idle (16 x 2400: 2.90 against 2.38 with one
+    // node per thread; 33 x 1300 2.44 against 2.41).
+    static constexpr int F32_NODE_CTAS = 3;
     static constexpr long long F32_NODE_MAX = 48000;
     int f32_form = 1;
     // FP64: k_fused at 128 registers (8 CTAs of 64 threads per SM, a few
@@ -235,7 +239,10 @@ struct Impl final : Solver {
         const long long nodes = (long long)p.nx * p.ny;
         const int pairs = split_ctas <= (long long)SPLIT_CTAS * n_sm && nodes <= SPLIT_MAX_NODES ? 2 : 1;
         if (is_p16<St>::value) kern = pairs;
-        f32_form = nodes <= F32_NODE_MAX ? 0 : pairs;
+        f32_form = (long long)grd.x * grd.y <= (long long)F32_NODE_CTAS * n_sm ? 0
+                   : pairs == 2                                                ? 2
+                   : nodes <= F32_NODE_MAX                                     ? 0
+                                                                               : 1;
         f64_packed = (long long)grd.x * grd.y > (long long)F64_CTAS * n_sm;
         if (!stream) {
             CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));

@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 
 SIZES = {
     "f32": [(4, 4), (33, 70), (96, 499), (97, 496), (128, 512), (101, 694), (129, 543), (130, 640),
-            (128, 546), (128, 547), (33, 1455), (33, 1500)],
+            (128, 546), (128, 547), (33, 1455), (33, 1500),
+            (128, 443), (128, 445), (98, 470), (20, 1100)],
     "f64": [(5, 4), (31, 63), (64, 32), (64, 33), (64, 443), (128, 443), (128, 445), (65, 593), (97, 601)],
 }
 
