@@ -393,29 +393,38 @@ CAV_OVER(over_2cs4, 0.5, I4H, I4L, A(2.0) * A(CS2) * A(CS2))
 // RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990, theorems on the
 // rounded reciprocal and quotient.  For b and a / b away from the ends of the
 // exponent range: here b is a density, a relaxation time or a fixed ratio of
-// order one; a numerator below 2^-900 may lose its last bit.  Infinite and NaN
-// quotients come out as a * y.  Checked against the division itself on 2^28
-// operand pairs (tests/test_gpu_quotient.py).  A compiled division checks its
-// range and branches, and code does not move across it.  B200, us per step with
-// divisions / with these: FP64 16 x 40 2.36 / 2.03, 64 x 256 2.54 / 2.16, 128 x 511
-// 4.52 / 4.30, the dynamic model on 64 x 256 8.52 / 8.02; the block-refined 64 x 256 in
-// three levels 40.3 / 37.2 per coarse step.
+// order one; a numerator below 2^-900 may lose its last bit.  Where b or a y is
+// zero, infinite or NaN the corrections are no numbers: the reciprocal is then
+// the approximation itself and the quotient a y, which are the division's
+// (an infinite turbulent Prandtl number: nu_t / Pr_t = 0).  Checked against the
+// division on 2^28 operand pairs (tests/test_gpu_quotient.py) and, bit for bit, on
+// those operands (tests/test_gpu_quotient_edges.py).  Code does not move across a
+// division's branch.  B200, us per step with divisions / with these: FP64 16 x 40
+// 2.36 / 2.03, 64 x 256 2.54 / 2.16, 128 x 511 4.52 / 4.30, the dynamic model on
+// 64 x 256 8.52 / 8.02; the block-refined 64 x 256 in three levels 40.3 / 37.2 per
+// coarse step (the same builds without the special operands: within 1 %).
 // ---------------------------------------------------------------------------
+// neither zero nor subnormal, infinite or NaN (an integer test: the FP64 pipe is
+// what the step waits for)
+__device__ __forceinline__ bool is_normal(double x) {
+    return unsigned(__double2hiint(x) & 0x7fffffff) - 0x00100000u < 0x7fe00000u;
+}
 __device__ __forceinline__ double rcp_rn(double b) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    const double e = __fma_rn(-b, y, 1.0);
+    const double y0 = y, e = __fma_rn(-b, y, 1.0);
     y = __fma_rn(y, __fma_rn(e, e, e), y);
     y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
     const bool ones = __double2loint(b) == -1 && (__double2hiint(b) | int(0xfff00000u)) == -1;
-    return __hiloint2double(__double2hiint(y), __double2loint(y) | (ones ? 1 : 0));
+    y = __hiloint2double(__double2hiint(y), __double2loint(y) | (ones ? 1 : 0));
+    return is_normal(b) ? y : y0;
 }
 // a / b from y = rcp_rn(b) (or the host's rounded 1 / b)
 __device__ __forceinline__ double quot_rn(double a, double b, double y) {
     const double q0 = __dmul_rn(a, y);
     const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
     const double q2 = __fma_rn(__fma_rn(-b, q1, a), y, q1);
-    return isfinite(q0) ? q2 : q0;
+    return is_normal(q0) ? q2 : q0;
 }
 
 // sqrt(x) without a branch: Newton steps on g = x y and h = y / 2 from the
