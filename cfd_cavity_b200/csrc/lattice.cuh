@@ -427,26 +427,35 @@ __device__ __forceinline__ double quot_rn(double a, double b, double y) {
     return is_normal(q0) ? q2 : q0;
 }
 
-// sqrt(x) without a branch: Newton steps on g = x y and h = y / 2 from the
-// special-function unit's y ~ 1 / sqrt(x) (Goldschmidt's coupled iteration as
-// in Markstein, above), then one exact-remainder correction, g + (x - g^2) h:
-// rounded as sqrt() but for the few x per binade whose root lies within
-// 2^-53 ulp of the middle of two numbers.  Zero, infinite and NaN x, and x below
-// 2^-960, come back as they are.  For the dynamic model's dozen independent roots
-// (64 x 256: 8.02 -> 7.52 us per step); the step itself has one, at the end of a
-// chain, where sqrt() is the shorter (2.05 us against 2.26 on 16 x 40).
+// sqrt(x) without a branch, for any x: Newton steps on g = x y and h = y / 2 from
+// the special-function unit's y ~ 1 / sqrt(x) (Goldschmidt's coupled iteration as
+// in Markstein, above), then one exact-remainder correction, g + (x - g^2) h.
+// Within one ulp, and rounded as sqrt() but for the few x per binade whose root
+// lies within 2^-53 ulp of the middle of two numbers
+// (tests/test_gpu_square_root.py).  An x below 2^-960 is taken 2^200 times larger
+// first, and its root 2^100 times smaller (exactly; the remainder must not leave
+// the normal numbers); zero and infinite x come back as they are, a negative one
+// as NaN.
+// For the dynamic model's dozen independent roots (64 x 256: 8.02 -> 7.52 us per
+// step); the step itself has one, at the end of a chain, where sqrt() is the
+// shorter (2.05 us against 2.26 on 16 x 40).
 __device__ __forceinline__ double sqrt_nr(double x) {
+    const int hi = __double2hiint(x);
+    const double xs = __dmul_rn(x, (hi & 0x7fffffff) < 63 << 20 ? 0x1p200 : 1.0);
     double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    double g = __dmul_rn(x, y), h = __dmul_rn(0.5, y);
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(xs));
+    double g = __dmul_rn(xs, y), h = __dmul_rn(0.5, y);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const double r = __fma_rn(-g, h, 0.5);
         g = __fma_rn(g, r, g);
         h = __fma_rn(h, r, h);
     }
-    g = __fma_rn(__fma_rn(-g, g, x), h, g);
-    return x >= 0x1p-960 && x <= 0x1p960 ? g : x;
+    g = __fma_rn(__fma_rn(-g, g, xs), h, g);
+    // (a NaN root stays one: only those of x >= 0 are scaled back)
+    const double root = __hiloint2double(__double2hiint(g) - (unsigned(hi) < 63u << 20 ? 100 << 20 : 0), __double2loint(g));
+    const int hs = __double2hiint(xs);  // (integer tests, as in is_normal)
+    return (hs & 0x7fffffff) == 0 || hs >= 0x7ff00000 ? x : root;
 }
 
 // ---------------------------------------------------------------------------

@@ -25,10 +25,12 @@
 // The default width of two nodes (eta_test = 2) has its windows unrolled
 // (WIDTH 2).  The uniform solver then runs the first two parts as one kernel
 // (k_sgs_bc2) and the third inside the collision (k_sgs_collide2).
-// Sums run in the reference's order (box windows row by row), so every
-// quantity but the a^alpha powers is bit-identical in FP64: CUDA's pow, within
-// 2 ulp of the reference's, or, at the default alpha = 1/2, one correctly
-// rounded square root of the product a b.
+// Sums run in the reference's order (box windows row by row).  In FP64 everything
+// but the roots and the a^alpha powers is then bit-identical.  The roots are
+// sqrt_nr's, within one ulp and rounded as sqrt() but for rare arguments; the
+// powers CUDA's pow, within 2 ulp of the reference's, or, at the default alpha =
+// 1/2, one such root of the product a b (zero where that product underflows: a
+// mixed form below 2^-537, lost beside any viscosity).
 #pragma once
 
 #include "kernels.cuh"
@@ -455,9 +457,10 @@ __global__ void __launch_bounds__(128) k_sgs_c(SgsGrids<St> S, Geom G, SgsParams
 
 // k_sgs_b and k_sgs_c in one for the test filter of two nodes: a node forms
 // qsm^1/2 and Phi_sm^1/2 of its window itself (three more square roots), so only
-// the six results go through memory and one launch is saved.
+// the six results go through memory and one launch is saved.  Held to 128 registers,
+// four CTAs per SM: with 138 the step on 128 x 512 took 14.8 us instead of 12.4.
 template <class St, bool HALF>
-__global__ void __launch_bounds__(128) k_sgs_bc2(SgsGrids<St> S, Geom G, SgsParams sp) {
+__global__ void __launch_bounds__(128, 4) k_sgs_bc2(SgsGrids<St> S, Geom G, SgsParams sp) {
     pdl_wait();
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
