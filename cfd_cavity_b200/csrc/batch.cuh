@@ -16,6 +16,7 @@
 // graphs of GRAPH_STEPS launches reading a device step counter.
 #pragma once
 
+#include "partition.h"
 #include "solver.cuh"
 #include "tile.cuh"
 #include "tilex.cuh"
@@ -55,15 +56,6 @@ constexpr int BATCH_THREADS = 128;
 // min(r, its spin-up), the last one (n_rows - 1 = the longest spin-up) the
 // steady state of all.
 __device__ __forceinline__ long long scalar_row(long long s, int n_rows) { return s < n_rows - 1 ? s : n_rows - 1; }
-// Largest state of the cavities stepped together (Batch::setup_groups).  The
-// 64-cavity sweep (2.29 M nodes: 340 MB in FP32, 175 MB in 16 bits) on a B200,
-// us per lattice step against the groups' size in MB:
-//   FP32  (k_batch_np)      340: 61.9   85: 52.5   68: 46.3   57: 46.0   42: 47.4
-//   f16sr (k_batch_x, r 2)  175: 48.6   87: 43.8   58: 40.0   44: 41.5   35: 42.6
-// Above ~70 MB a group's planes push each other out of the 126 MB L2; small
-// groups pay each launch's start and last wave over fewer nodes.
-constexpr size_t GROUP_BYTES = 75'000'000;
-
 template <class St, bool WRITE_NUT>
 __global__ void __launch_bounds__(BATCH_THREADS)
     k_batch(const BatchCav<St>* __restrict__ cavs, const BatchItem* __restrict__ items, int n_items,
@@ -297,23 +289,15 @@ struct Batch final : BatchBase {
     }
 
     // The cavities are independent, so a call's steps are run for one group of
-    // them after another, each group small enough that its state stays in the
-    // L2 from step to step (126 MB; the rest is left to what else passes
-    // through), and about equal in size.
+    // them after another, cut so that a group's state stays in the L2 from step to
+    // step where the cavities' sizes allow it (partition.h).
     void setup_groups() {
-        auto bytes = [&](const Impl<St>* c) { return c->field_elems() * (2 * NPLANES * sizeof(St) + sizeof(A)); };
-        size_t total = 0;
-        for (auto* c : cv) total += bytes(c);
-        const size_t n = (total + GROUP_BYTES - 1) / GROUP_BYTES;
-        size_t done = 0, last = 0;
-        for (int i = 0; i < int(cv.size()); ++i) {
-            // a cavity goes with the group that its middle lies in
-            const size_t g = std::min(n - 1, (done + bytes(cv[i]) / 2) * n / total);
-            if (groups.empty() || g != last) groups.push_back(Group{i, i});
-            last = g;
-            groups.back().c1 = i + 1;
-            done += bytes(cv[i]);
-        }
+        int l2 = 0;
+        CK(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, cv[0]->p.device));
+        std::vector<size_t> bytes;
+        for (auto* c : cv) bytes.push_back(c->field_elems() * (2 * NPLANES * sizeof(St) + sizeof(A)));
+        const std::vector<int> first = partition_groups(bytes, size_t(l2));
+        for (size_t i = 0; i + 1 < first.size(); ++i) groups.push_back(Group{first[i], first[i + 1]});
     }
 
     // First item of every cavity (and the number of items) in a cavity-major list.
