@@ -1,6 +1,6 @@
 """Python mirror of the batch C ABI (``cav_batch_*``): many cavities advanced
-together, one kernel launch per lattice step and per group of cavities whose
-state fits the L2.
+together, one kernel launch per lattice step over all of them or per group of
+cavities whose state fits the L2.
 
 The reference runs one cavity per process (``src/main.rs:42-443``); a batch
 is a set of ``CavitySolver::new`` objects stepped together.  Each cavity of a

@@ -7,9 +7,10 @@
 // `rows`-row) tiles: grid = ctas_per_sm x #SMs CTAs of 128 threads that
 // stride over the list.  Tiles are ordered cavity-major, row-block-minor, so
 // the tiles in flight at one time are neighbours and the halo rows they
-// share are served by L2.  A call's steps run group of cavities by group
-// (setup_groups), so that a group's state stays in the L2 between its steps.  Per-cavity step scalars (ramps, seeds, wall
-// temperature pointers) come from a device table precomputed on the host with
+// share are served by L2.  Where that pays (ungrouped_steps), a call's steps run
+// group of cavities by group (setup_groups), so that a group's state stays in the
+// L2 between its steps.  Per-cavity step scalars (ramps, seeds, wall temperature
+// pointers) come from a device table precomputed on the host with
 // the single-cavity code (Impl::scalars), row min(step, spin_up), and every
 // node runs the same fused_node() as k_fused: a cavity advanced in a batch
 // is bit-identical to the same cavity advanced alone.  Steps run as CUDA
@@ -21,6 +22,8 @@
 #include "tile.cuh"
 #include "tilex.cuh"
 #include "xpair.cuh"
+
+#include <limits>
 
 namespace cav {
 
@@ -222,6 +225,7 @@ struct Batch final : BatchBase {
         cudaGraphExec_t graph = nullptr;
     };
     std::vector<Group> groups;
+    Group every{0, 0};  // all cavities at once (calls that are too short for groups)
     bool cavs_dirty = true;
     // the tile kernel (tile.cuh)
     TileCav<St>* d_tcavs = nullptr;
@@ -239,8 +243,7 @@ struct Batch final : BatchBase {
     bool stall_copies = false;  // test of the bounded waits: arm the barriers, issue no copy
 
     ~Batch() override {
-        for (Group& g : groups)
-            if (g.graph) cudaGraphExecDestroy(g.graph);
+        drop_graphs();
         if (h_err) cudaFreeHost(h_err);
         void* bufs[] = {d_cavs,      d_items, d_work,     d_table, step_dev, d_tcavs,   d_maps[1],
                         d_maps[2],   d_titems[1], d_titems[2], d_err,  d_xmaps[0],
@@ -298,6 +301,7 @@ struct Batch final : BatchBase {
         for (auto* c : cv) bytes.push_back(c->field_elems() * (2 * NPLANES * sizeof(St) + sizeof(A)));
         const std::vector<int> first = partition_groups(bytes, size_t(l2));
         for (size_t i = 0; i + 1 < first.size(); ++i) groups.push_back(Group{first[i], first[i + 1]});
+        every.c1 = first.back();
     }
 
     // First item of every cavity (and the number of items) in a cavity-major list.
@@ -433,17 +437,19 @@ struct Batch final : BatchBase {
             g.item0 = first[g.c0];
             g.n_items = first[g.c1] - first[g.c0];
         }
+        every.n_items = first[every.c1];
         work_dirty = true;
         drop_graphs();
         CK(cudaStreamSynchronize(stream));
     }
 
     void drop_graphs() {
-        for (Group& g : groups)
-            if (g.graph) {
-                cudaGraphExecDestroy(g.graph);
-                g.graph = nullptr;
-            }
+        auto drop = [](Group& g) {
+            if (g.graph) cudaGraphExecDestroy(g.graph);
+            g.graph = nullptr;
+        };
+        for (Group& g : groups) drop(g);
+        drop(every);
     }
 
     // Brings every cavity to PC form at the shared step and refreshes the
@@ -632,8 +638,38 @@ struct Batch final : BatchBase {
         enter();  // may run one collision (the first step from a REF state)
         if (entered_with_collide) n -= 1;
         if (n <= 0) return;
-        for (Group& g : groups) step_group(g, n);
+        if (groups.size() > 1 && n > ungrouped_steps()) {
+            for (Group& g : groups) step_group(g, n);
+        } else {
+            step_group(every, n);
+        }
         advance_cavities(n);
+    }
+
+    // The longest call that is run as one launch per step over all cavities.  A
+    // group pays a launch's start and last wave at every step and gains from its
+    // second step on, and only where the kernel waits for memory: the TMA-staged
+    // kernels (1, 6; 2 in 16 bits) and the one-node kernel 3 in 16 bits, which is
+    // bound by issue, do not.  B200, us per step of an n-step call, one launch /
+    // groups (64-cavity sweep; 160 cavities):
+    //   FP32 kernel 3    n 1: 80.0 / 93.2   2: 71.3 / 75.0   3: 66.5 / 62.9   (160) 2: 169 / 179   3: 164 / 158
+    //   f16sr kernel 5   n 1: 71.4 / 69.2   2: 54.1 / 56.5   3: 52.2 / 51.9   (160) 2: 127 / 137   3: 125 / 127
+    //   f16sr kernel 4   n 3: 56.4 / 56.3   6: 52.7 / 51.9   64: 49.5 / 47.6  (160) 4: 132 / 139   16: 128 / 130
+    //   f16sr kernel 3   n 1: 76.9 / 80.6   8: 53.6 / 55.5   64: 51.2 / 52.2  (160) 64: 135 / 139
+    //   f16sr kernel 6   n 1: 65.8 / 73.8   8: 44.1 / 49.7   64: 42.1 / 45.8  (160) 64: 113 / 122
+    //   FP32 kernel 0    n 8: 78.9 / 80.5   16: 77.8 / 77.0  64: 77.1 / 74.5  (160) 16: 194 / 195
+    //   FP32 kernel 2    n 4: 101 / 102     8: 99.6 / 93.0   64: 98.5 / 85.6  (160) 6: 243 / 242
+    int64_t ungrouped_steps() const {
+        constexpr bool p16 = is_p16<St>::value;
+        constexpr int64_t any = std::numeric_limits<int64_t>::max();
+        switch (effective_kernel(tun.kernel)) {
+            case 0: return 16;
+            case 2: return p16 ? any : 6;
+            case 3: return p16 ? any : 2;
+            case 4: return p16 ? 4 : 2;
+            case 5: return 2;
+            default: return any;
+        }
     }
 
     // n steps of one group from the shared step (its cavities in PC form).

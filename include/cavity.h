@@ -303,7 +303,9 @@ const char* cav_batch_last_error(const cav_batch* b);
 /* n steps of every cavity.  Cavities are independent, so a batch whose state
  * is larger than the L2 advances in groups of consecutive cavities, cut so that
  * a group's state stays in the L2 where the cavities' sizes allow it, each group
- * taking all n steps before the next (one kernel launch per group and step). */
+ * taking all n steps before the next (one kernel launch per group and step).
+ * Calls of a few steps, and kernels that gain nothing from it, run one launch per
+ * step over all cavities. */
 int cav_batch_step(cav_batch* b, int64_t n);
 int cav_batch_get_fields(cav_batch* b, int32_t i, double* rho, double* ux, double* uy, double* t,
                          double* nu_t, double* fy);
