@@ -197,7 +197,9 @@ __device__ __forceinline__ void pull_g_channel(const St* __restrict__ src, const
     }
 }
 
-template <class St, bool LANE = false>
+// SELECT: the wall's value is chosen beside each load, not after all of them, and
+// the loads then come in several rounds (where that pays: Impl::f32_form).
+template <class St, bool LANE = false, bool SELECT = false>
 __device__ __forceinline__ void pull_g(const St* __restrict__ src, const Geom& G, int ix, int iy,
                                        const StepScalars<typename Fmt<St>::A>& c, typename Fmt<St>::A (&g)[Q]) {
     using A = typename Fmt<St>::A;
@@ -213,21 +215,22 @@ __device__ __forceinline__ void pull_g(const St* __restrict__ src, const Geom& G
         // wall columns read their own node (a valid address) and discard it
         const int idx = (Q + i) * P + (wall_col ? kg : kg - CX(i) - CY(i) * W);
         g[i] = LANE ? Fmt<St>::lload(src[idx], Q + i) : Fmt<St>::load(src[idx], Q + i);
+        if (SELECT && wall_col) g[i] = geq_rest<A>(i, tw, c.geq_order);
     }
     // after all the loads: a select beside each load lets the compiler put
     // the load under the wall-column branch, one round trip after another
-    if (wall_col) {
+    if (!SELECT && wall_col) {
 #pragma unroll
         for (int i = 0; i < Q; ++i) g[i] = geq_rest<A>(i, tw, c.geq_order);
     }
 }
 
-template <class St, bool LANE = false>
+template <class St, bool LANE = false, bool SELECT = false>
 __device__ __forceinline__ void pull_node(const St* __restrict__ src, const Geom& G, int ix, int iy,
                                           const StepScalars<typename Fmt<St>::A>& c,
                                           typename Fmt<St>::A (&f)[Q], typename Fmt<St>::A (&g)[Q]) {
     pull_f<St, LANE>(src, G, ix, iy, f);
-    pull_g<St, LANE>(src, G, ix, iy, c, g);
+    pull_g<St, LANE, SELECT>(src, G, ix, iy, c, g);
 }
 
 // Temperature of node (ix, iy) of the streamed state, gathered from a PC
@@ -329,7 +332,7 @@ __device__ __forceinline__ void fused_core(typename Fmt<St>::A (&f)[Q], typename
     store_node<St, true>(dst, G, iy, ix, f, g, c);
 }
 
-template <class St, bool WRITE_NUT, bool ACC_NU, bool NO_COLLIDE, bool CHANNEL = false>
+template <class St, bool WRITE_NUT, bool ACC_NU, bool NO_COLLIDE, bool CHANNEL = false, bool SELECT = false>
 __device__ __forceinline__ void fused_node_io(const St* __restrict__ src, St* __restrict__ dst,
                                               const typename Fmt<St>::A* fy_in, typename Fmt<St>::A* fy_out,
                                               typename Fmt<St>::A* __restrict__ nut, double* __restrict__ acc_hot,
@@ -341,20 +344,20 @@ __device__ __forceinline__ void fused_node_io(const St* __restrict__ src, St* __
         pull_f<St, true, true>(src, G, ix, iy, f);
         pull_g_channel<St, true>(src, G, ix, iy, g);
     } else {
-        pull_node<St, true>(src, G, ix, iy, c, f, g);
+        pull_node<St, true, SELECT>(src, G, ix, iy, c, f, g);
     }
     auto t_at = [&](int x) { return gather_t<St>(src, G, x, iy, c); };
     fused_core<St, WRITE_NUT, ACC_NU && !CHANNEL, NO_COLLIDE, decltype(t_at)&, CHANNEL>(
         f, g, dst, fy_in, fy_out, nut, acc_hot, acc_cold, G, ix, iy, c, t_at);
 }
 
-template <class St, bool WRITE_NUT, bool ACC_NU, bool NO_COLLIDE, bool CHANNEL = false>
+template <class St, bool WRITE_NUT, bool ACC_NU, bool NO_COLLIDE, bool CHANNEL = false, bool SELECT = false>
 __device__ __forceinline__ void fused_node(const St* __restrict__ src, St* __restrict__ dst,
                                            typename Fmt<St>::A* fy, typename Fmt<St>::A* __restrict__ nut,
                                            double* __restrict__ acc_hot, double* __restrict__ acc_cold,
                                            const Geom& G, int ix, int iy, const StepScalars<typename Fmt<St>::A>& c) {
-    fused_node_io<St, WRITE_NUT, ACC_NU, NO_COLLIDE, CHANNEL>(src, dst, fy, fy, nut, acc_hot, acc_cold, G, ix, iy,
-                                                              c);
+    fused_node_io<St, WRITE_NUT, ACC_NU, NO_COLLIDE, CHANNEL, SELECT>(src, dst, fy, fy, nut, acc_hot, acc_cold, G, ix,
+                                                                      iy, c);
 }
 
 // Two nodes of one column, (ix, iy) and (ix, iy + 1), in one thread: the
@@ -440,7 +443,7 @@ __device__ __forceinline__ void fused_pair(const St* __restrict__ src, St* __res
 //              test of the TRT + Guo collision, src/uniform/tests.rs:246-376,
 //              turned by 90 degrees).
 template <class St, bool WRITE_NUT, bool ACC_NU, bool NO_COLLIDE, bool CHANNEL = false, int THREADS = 256,
-          int MIN_CTAS = 1>
+          int MIN_CTAS = 1, bool SELECT = false>
 __global__ void __launch_bounds__(THREADS, MIN_CTAS) k_fused(const St* __restrict__ src, St* __restrict__ dst,
                                                              typename Fmt<St>::A* __restrict__ fy,
                                                              typename Fmt<St>::A* __restrict__ nut,
@@ -451,7 +454,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) k_fused(const St* __restric
     const int ix = blockIdx.x * blockDim.x + threadIdx.x;
     const int iy = blockIdx.y * blockDim.y + threadIdx.y;
     if (ix >= G.nx || iy >= G.ny) return;
-    fused_node<St, WRITE_NUT, ACC_NU, NO_COLLIDE, CHANNEL>(src, dst, fy, nut, acc_hot, acc_cold, G, ix, iy, c);
+    fused_node<St, WRITE_NUT, ACC_NU, NO_COLLIDE, CHANNEL, SELECT>(src, dst, fy, nut, acc_hot, acc_cold, G, ix, iy, c);
 }
 
 // collide(step) on a REF state (populations + fields), writing PC to dst.

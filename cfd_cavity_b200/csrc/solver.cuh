@@ -184,17 +184,26 @@ struct Impl final : Solver {
     static constexpr int SPLIT_CTAS = 4;
     static constexpr long long SPLIT_MAX_NODES = 70000;
     int kern = is_p16<St>::value ? 1 : 0;
-    // FP32 (step kernel 0): one node per thread while three CTAs per SM hold the
-    // grid (one thread's chain is all there is: 96 x 384 1.80 us per step against
-    // 1.96 for split pairs; 126 x 386 2.18 against 2.28), pairs split over two
-    // warps while those run at once (128 x 512 2.19 against 2.40, 98 x 470 2.19
-    // against 2.36), and past that plain pairs (130 x 530: 2.59 against 3.21 split;
-    // 512 x 1024: 8.8 against 9.2, one node per thread 11.6) unless the grid is
-    // narrow, where they leave most lanes idle (16 x 2400: 2.90 against 2.38 with one
-    // node per thread; 33 x 1300 2.44 against 2.41).
-    static constexpr int F32_NODE_CTAS = 3;
-    static constexpr long long F32_NODE_MAX = 48000;
-    int f32_form = 1;
+    // FP32 (step kernel 0), by the CTAs per SM of one node per thread (128 threads,
+    // all of up to 8 at once) and of plain pairs (64 threads, 10 at once); B200, us
+    // per step of one node / one node with its loads in rounds / pairs split over
+    // two warps / plain pairs:
+    //   up to 3 one-node CTAs: one node per thread, one chain, every load at once
+    //     (64 x 512 1.67 / 1.70 / 1.74 / 1.80; 110 x 440 2.06 / 2.15 / 2.22 / 2.19);
+    //   up to 4.5: the same with its loads in rounds (k_fused SELECT): that many warps
+    //     queue for the L2 with every load at once (72 x 620 2.32 / 2.21 / 2.70 / 2.43;
+    //     128 x 512 2.40 / 2.22 / 2.21 / 2.31; 256 x 270 2.47 / 2.22 / 2.32 / 2.38;
+    //     130 x 530 2.65 / 2.55 / 3.18 / 2.60);
+    //   above, plain pairs (33 x 2000 3.14 / 3.19 / - / 2.76; 256 x 700 4.00 / 4.08 / - /
+    //     3.62; 480 x 1500 16.9 / 17.7 / - / 15.9), but one node per thread where a third
+    //     or more of the pairs' lanes would lie beyond the right wall (1 or 3 columns
+    //     of 32: 24 x 2600 2.47 / 2.51 / - / 2.92; 96 x 2000 4.10 / 4.20 / - / 4.57; 32 x
+    //     12000 6.86 / 6.85 / - / 9.26) and where the pairs are somewhat more than one
+    //     wave (512 x 400 4.20 / 4.32 / - / 4.46; 224 x 1000 4.50 / 4.53 / - / 4.77; from 13
+    //     one-node CTAs on level again: 512 x 512 5.13 / 5.10 / - / 5.04).
+    static constexpr int F32_ONE_ROUND_CTAS = 3, F32_ROUNDS_CTAS_X2 = 9, F32_PAIR_WAVE_CTAS = 10, F32_PAIR_CTAS = 13;
+    enum { F32_NODE = 0, F32_PAIR = 1, F32_NODE_ROUNDS = 3 };
+    int f32_form = F32_NODE;
     // FP64: k_fused at 128 registers (8 CTAs of 64 threads per SM, a few
     // words spilled) once the grid is more than the one wave that its 156
     // registers leave room for (6 per SM): 128 x 511, 1024 CTAs, 4.50 us per
@@ -239,10 +248,16 @@ struct Impl final : Solver {
         const long long nodes = (long long)p.nx * p.ny;
         const int pairs = split_ctas <= (long long)SPLIT_CTAS * n_sm && nodes <= SPLIT_MAX_NODES ? 2 : 1;
         if (is_p16<St>::value) kern = pairs;
-        f32_form = (long long)grd.x * grd.y <= (long long)F32_NODE_CTAS * n_sm ? 0
-                   : pairs == 2                                                ? 2
-                   : nodes <= F32_NODE_MAX                                     ? 0
-                                                                               : 1;
+        const long long node_ctas = (long long)grd.x * grd.y, pair_ctas = (long long)grdx.x * grdx.y;
+        if (node_ctas <= (long long)F32_ONE_ROUND_CTAS * n_sm)
+            f32_form = F32_NODE;
+        else if (2 * node_ctas <= (long long)F32_ROUNDS_CTAS_X2 * n_sm)
+            f32_form = F32_NODE_ROUNDS;
+        else if (nbx != 1 && nbx != 3 &&
+                 (pair_ctas <= (long long)F32_PAIR_WAVE_CTAS * n_sm || node_ctas > (long long)F32_PAIR_CTAS * n_sm))
+            f32_form = F32_PAIR;
+        else
+            f32_form = F32_NODE;
         f64_packed = (long long)grd.x * grd.y > (long long)F64_CTAS * n_sm;
         if (!stream) {
             CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
@@ -447,11 +462,20 @@ struct Impl final : Solver {
                                       nut, acc_hot, acc_cold, G, c));
                 return;
             }
+        }
+        if constexpr (is_p16<St>::value) {
             if (form() == 2) {
                 cfg.gridDim = dim3(((p.nx + 1) / 2 + 31) / 32, (p.ny + XS_ROWS - 1) / XS_ROWS);
                 cfg.blockDim = dim3(64 * XS_ROWS);
                 CK(cudaLaunchKernelEx(&cfg, k_fused_xs<St, WN, ACC>, (const St*)pop[cur], pop[cur ^ 1], fy, nut,
                                       acc_hot, acc_cold, G, c));
+                return;
+            }
+        }
+        if constexpr (std::is_same<St, float>::value) {
+            if (form() == F32_NODE_ROUNDS) {
+                CK(cudaLaunchKernelEx(&cfg, k_fused<St, WN, ACC, false, false, 256, 1, true>, (const St*)pop[cur],
+                                      pop[cur ^ 1], fy, nut, acc_hot, acc_cold, G, c));
                 return;
             }
         }
@@ -808,8 +832,15 @@ struct Impl final : Solver {
                 for (int64_t j = 0; j < step_arg; ++j) {
                     bool done = false;
                     if constexpr (has_pairs<St>::value) {
-                        if (form() >= 1) {
+                        if (form() == 1 || form() == 2) {
                             k_fused_x<St, false, false, true><<<grdx, blkx, 0, stream>>>(
+                                pop[cur], pop[cur ^ 1], fy, nut, acc_hot, acc_cold, G, scalars(time_step));
+                            done = true;
+                        }
+                    }
+                    if constexpr (std::is_same<St, float>::value) {
+                        if (form() == F32_NODE_ROUNDS) {
+                            k_fused<St, false, false, true, false, 256, 1, true><<<grd, blk, 0, stream>>>(
                                 pop[cur], pop[cur ^ 1], fy, nut, acc_hot, acc_cold, G, scalars(time_step));
                             done = true;
                         }
