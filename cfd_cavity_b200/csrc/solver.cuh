@@ -489,8 +489,8 @@ struct Impl final : Solver {
         CK(cudaLaunchKernelEx(&cfg, k_fused<St, WN, ACC, false>, (const St*)pop[cur], pop[cur ^ 1], fy, nut,
                               acc_hot, acc_cold, G, c));
     }
-    // The kernel that runs a step: set_step_kernel's choice for the 16-bit
-    // formats; FP32 takes the node-pair kernels by size, FP64 one node per thread.
+    // The kernel that runs a step: kern for the 16-bit formats, f32_form for FP32
+    // (both set by size until set_step_kernel), one node per thread for FP64.
     int form() const {
         return is_p16<St>::value ? kern : (std::is_same<St, float>::value ? f32_form : 0);
     }
@@ -501,6 +501,7 @@ struct Impl final : Solver {
             throw ArgError{CAV_ERR_ARG, "the node-pair step kernel is for the 16-bit storage formats"};
         CK(cudaStreamSynchronize(stream));
         kern = k;
+        f32_form = F32_NODE;  // FP32: the caller's choice instead of the rule's
         for (auto& row : graph)
             for (auto& gx : row)
                 if (gx) {

@@ -168,7 +168,7 @@ class CavitySolver:
         nodes per thread, 2 the same pairs with their f and g halves on two
         warps (16-bit formats: 2 is the default up to 70 000 nodes while
         all its blocks run at once, else 1; FP32 reports 0 and chooses by
-        size itself); same bits."""
+        size itself until 0 is set here); same bits."""
         self._ck(L.load().cav_set_step_kernel(self._h, int(kernel)))
 
     def step_kernel(self):

@@ -201,7 +201,7 @@ int cav_launch_count(cav_handle* h, int64_t* n);
  * CAV_STEP_PAIR_SPLIT up to 70 000 nodes while all its blocks of 64 x 2 nodes
  * run at once (four per SM), CAV_STEP_PAIR otherwise; FP64 / FP32:
  * CAV_STEP_NODE, with which FP32 takes the library's own choice by size between
- * one node per thread and node pairs.  All give the same bits; CAV_ERR_ARG for a pair kernel on
+ * one node per thread and node pairs until CAV_STEP_NODE is set by the caller.  All give the same bits; CAV_ERR_ARG for a pair kernel on
  * FP64 / FP32. */
 #define CAV_STEP_NODE 0
 #define CAV_STEP_PAIR 1

@@ -48,3 +48,15 @@ def test_nusselt_sums_of_the_rounds_form():
         want += [np.abs(p[:, 1] - p[:, 2]).mean(), np.abs(p[:, -2] - p[:, -3]).mean()]
     # FP64 sums of the same FP32 temperatures, in another order
     assert np.allclose([hot, cold], want / 6 * (ny - 1), rtol=1e-12, atol=0)
+
+
+@pytest.mark.parametrize("nx,ny", [(129, 356), (255, 739)])  # rounds, pairs
+def test_one_node_per_thread_when_the_caller_sets_it(nx, ny):
+    s, t = (CavitySolver(nx, ny, 1e6, 0.71, 0.1, 0.9, 0.02, 3, precision="f32") for _ in range(2))
+    s.step(280)  # past the ramp: graphs of the rule's kernel
+    s.set_step_kernel(L.CAV_STEP_NODE)
+    assert s.step_kernel() == L.CAV_STEP_NODE
+    s.step(90)
+    t.step(370)
+    for p, q in zip(s.populations(), t.populations()):
+        np.testing.assert_array_equal(p, q)
