@@ -973,7 +973,7 @@ struct Impl final : Solver {
             St* ck_pop = nullptr;
             A *ck_fy = nullptr, *P[2] = {nullptr, nullptr};
             double *acc_cs_d = nullptr, *acc_th_d = nullptr;
-            cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
+            cudaEvent_t ev[4] = {};  // forward begins, ends; reverse begins, ends
             struct Free {
                 std::vector<void*> v;
                 ~Free() {
@@ -1004,7 +1004,7 @@ struct Impl final : Solver {
             struct Ev {
                 cudaEvent_t* e;
                 ~Ev() {
-                    for (int i = 0; i < 3; ++i)
+                    for (int i = 0; i < 4; ++i)
                         if (e[i]) cudaEventDestroy(e[i]);
                 }
             } evg{ev};
@@ -1037,8 +1037,11 @@ struct Impl final : Solver {
             // by side.  Events order the reuse of a slot set.  Each stream has
             // its own device step counter; full segments (length C, even) past
             // the ramps are CUDA graphs, one pair per slot set, with the steady
-            // scalars in their launches; the others are launched step by step
-            // with the scalars of the table.
+            // scalars in their launches; the others, a few ramp segments and the
+            // last one, are launched step by step with the scalars of the table
+            // (graphs of their own cost the host more than they save: 96 x 384
+            // FP32, 300 steps with 50 per segment, 8.4 ms a call without and 10.0
+            // with them).
             long long* sd_rec = sdev2;
             long long* sd_adj = sdev2 + 1;
             cudaStream_t rs = nullptr, hs = nullptr;
@@ -1207,6 +1210,7 @@ struct Impl final : Solver {
                 cp = (use_graphs && L_last != C && (L_last & 1)) ? 1 : 0;
             }
             CK(cudaStreamWaitEvent(hs, ev[1], 0));
+            CK(cudaEventRecord(ev[2], hs));  // (not ev[1]: the host may still have built graphs since)
             k_adj_final<St><<<grd, blk, 0, hs>>>(pop[cur], P[cp], G, scalars(N), obj, N);
             check_launch();
             CK(cudaStreamWaitEvent(rs, ev[1], 0));  // checkpoints complete
@@ -1215,8 +1219,8 @@ struct Impl final : Solver {
                 if (k >= 1) recompute(k - 1);
                 sweep(k);
             }
-            CK(cudaEventRecord(ev[2], hs));
-            CK(cudaStreamWaitEvent(stream, ev[2], 0));
+            CK(cudaEventRecord(ev[3], hs));
+            CK(cudaStreamWaitEvent(stream, ev[3], 0));
             CK(cudaStreamSynchronize(hs));
             CK(cudaStreamDestroy(hs));
             hs = nullptr;
@@ -1234,7 +1238,7 @@ struct Impl final : Solver {
             }
             float ms_f = 0.f, ms_r = 0.f;
             CK(cudaEventElapsedTime(&ms_f, ev[0], ev[1]));
-            CK(cudaEventElapsedTime(&ms_r, ev[1], ev[2]));
+            CK(cudaEventElapsedTime(&ms_r, ev[2], ev[3]));
             out[0] = J;
             out[1] = gcs;
             out[2] = ms_f;
