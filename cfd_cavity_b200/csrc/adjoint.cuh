@@ -85,7 +85,7 @@ __global__ void k_adj_final(const St* __restrict__ X, typename Fmt<St>::A* __res
 }
 
 // Step scalars of step s: from the per-step table (rows 0..S, row S = steady
-// state), or, with every step of the sweep in the steady state (S < 0), given
+// state), or, with every step of the sweep in the steady state (STEADY), given
 // with the launch: the table's row is a memory round trip after the step
 // counter's and the wall temperatures a third one after it, at the start of
 // every step (96 x 384 FP32 on a B200: reverse step 4.42 -> 4.20 us).

@@ -208,7 +208,7 @@ struct Batch final : BatchBase {
     using A = typename Fmt<St>::A;
     std::vector<Impl<St>*> cv;
     BatchCav<St>* d_cavs = nullptr;
-    BatchItem* d_items = nullptr;
+    BatchItem* d_items = nullptr;     // the items of kernel 0
     BatchWork<St>* d_work = nullptr;  // the items of kernels 3, 4 and 5 with their cavities
     std::vector<BatchItem> items;     // the current kernel's work list
     std::vector<BatchCav<St>> hcavs;  // host copy of d_cavs
@@ -419,9 +419,12 @@ struct Batch final : BatchBase {
                 for (int x0 = 0; x0 < nx; x0 += width) items.push_back({i, x0, y0, std::min(r, ny - y0)});
         }
         if (d_items) CK(cudaFree(d_items));
-        CK(cudaMalloc(&d_items, sizeof(BatchItem) * items.size()));
-        CK(cudaMemcpyAsync(d_items, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice,
-                           stream));
+        d_items = nullptr;
+        if (k == 0) {
+            CK(cudaMalloc(&d_items, sizeof(BatchItem) * items.size()));
+            CK(cudaMemcpyAsync(d_items, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice,
+                               stream));
+        }
         occ = tun.ctas_per_sm;  // the persistent kernel 0: as asked
         std::vector<int> first;
         if (k == 1 || k == 2) {
@@ -534,7 +537,7 @@ struct Batch final : BatchBase {
                               int(stall_copies)));
     }
 
-    // The one-CTA-per-item kernels (3, 4, 5) over d_items.
+    // The one-CTA-per-item kernels (3, 4, 5) over d_work.
     template <bool WN>
     void launch_np(const Group& g, int k, const long long* sdev, long long step) {
         const BatchWork<St>* const work = d_work + g.item0;

@@ -215,13 +215,13 @@ __device__ __forceinline__ void pull_g(const St* __restrict__ src, const Geom& G
         // wall columns read their own node (a valid address) and discard it
         const int idx = (Q + i) * P + (wall_col ? kg : kg - CX(i) - CY(i) * W);
         g[i] = LANE ? Fmt<St>::lload(src[idx], Q + i) : Fmt<St>::load(src[idx], Q + i);
-        if (SELECT && wall_col) g[i] = geq_rest<A>(i, tw, c.geq_order);
+        if (SELECT && wall_col) g[i] = geq_rest<A>(i, tw);
     }
     // after all the loads: a select beside each load lets the compiler put
     // the load under the wall-column branch, one round trip after another
     if (!SELECT && wall_col) {
 #pragma unroll
-        for (int i = 0; i < Q; ++i) g[i] = geq_rest<A>(i, tw, c.geq_order);
+        for (int i = 0; i < Q; ++i) g[i] = geq_rest<A>(i, tw);
     }
 }
 
@@ -243,10 +243,10 @@ __device__ __forceinline__ typename Fmt<St>::A gather_t(const St* __restrict__ s
     A g[Q];
     if (ix == 0) {
 #pragma unroll
-        for (int i = 0; i < Q; ++i) g[i] = geq_rest<A>(i, c.t_hot[gy], c.geq_order);
+        for (int i = 0; i < Q; ++i) g[i] = geq_rest<A>(i, c.t_hot[gy]);
     } else if (ix == G.nx - 1) {
 #pragma unroll
-        for (int i = 0; i < Q; ++i) g[i] = geq_rest<A>(i, c.t_cold, c.geq_order);
+        for (int i = 0; i < Q; ++i) g[i] = geq_rest<A>(i, c.t_cold);
     } else {
 #pragma unroll
         for (int i = 0; i < Q; ++i) g[i] = ldp(src, G, Q + i, gy - CY(i), ix - CX(i));
@@ -713,8 +713,8 @@ __global__ void k_dbg_thermal_v(St* __restrict__ pop, Geom G, StepScalars<typena
     if (iy >= G.ny) return;
 #pragma unroll
     for (int i = 0; i < Q; ++i) {
-        stp(pop, G, Q + i, iy, 0, geq_rest<A>(i, c.t_hot[iy], c.geq_order));
-        stp(pop, G, Q + i, iy, G.nx - 1, geq_rest<A>(i, c.t_cold, c.geq_order));
+        stp(pop, G, Q + i, iy, 0, geq_rest<A>(i, c.t_hot[iy]));
+        stp(pop, G, Q + i, iy, G.nx - 1, geq_rest<A>(i, c.t_cold));
     }
 }
 // ... then the horizontal walls copy rows 1 and ny-2.

@@ -941,7 +941,7 @@ __device__ __forceinline__ void collide_node_lane(L (&f)[Q], L (&g)[Q], const Ma
 // src/uniform/solver.rs:957-970): geq(T_wall, 0, 0) = w_i T_wall.
 // (The bracket of geq_full is 1 at u = 0 in either order.)
 template <class A>
-__device__ __forceinline__ A geq_rest(int i, A t, int) {
+__device__ __forceinline__ A geq_rest(int i, A t) {
     return A(WD(i)) * t;
 }
 

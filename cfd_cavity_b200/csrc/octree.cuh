@@ -502,7 +502,7 @@ __device__ __forceinline__ void bc_g(const LvlIO<St>& L, int x, int y, const Src
     }
     if (wall) {
 #pragma unroll
-        for (int i = 0; i < Q; ++i) g[i] = geq_rest<A>(i, tw, 2);
+        for (int i = 0; i < Q; ++i) g[i] = geq_rest<A>(i, tw);
     } else {
         const Src r = (xs == x && ys == y) ? own : src_of<COARSE>(L, xs, ys);
 #pragma unroll

@@ -140,7 +140,7 @@ __device__ __forceinline__ void pull_tile(const St* __restrict__ S, const Geom& 
         const int off = wall_col ? ((Q + i) * BY + row) * TILE_BX + col
                                  : ((Q + i) * BY + grow - CY(i)) * TILE_BX + col - CX(i);
         const A v = Fmt<St>::lload(S[off], Q + i);
-        g[i] = wall_col ? geq_rest<A>(i, tw, c.geq_order) : v;
+        g[i] = wall_col ? geq_rest<A>(i, tw) : v;
     }
 }
 
@@ -155,10 +155,10 @@ __device__ __forceinline__ typename Fmt<St>::A tile_t(const St* __restrict__ S, 
     A g[Q];
     if (x == 0) {
 #pragma unroll
-        for (int i = 0; i < Q; ++i) g[i] = geq_rest<A>(i, c.t_hot[gy], c.geq_order);
+        for (int i = 0; i < Q; ++i) g[i] = geq_rest<A>(i, c.t_hot[gy]);
     } else if (x == G.nx - 1) {
 #pragma unroll
-        for (int i = 0; i < Q; ++i) g[i] = geq_rest<A>(i, c.t_cold, c.geq_order);
+        for (int i = 0; i < Q; ++i) g[i] = geq_rest<A>(i, c.t_cold);
     } else {
 #pragma unroll
         for (int i = 0; i < Q; ++i) g[i] = tile_at<St, BY>(S, Q + i, grow - CY(i), col_x - CX(i));
