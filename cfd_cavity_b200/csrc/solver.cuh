@@ -163,12 +163,14 @@ struct Impl final : Solver {
     cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
     // Block height of the one-node kernels: 32 x 4 for FP32 storage, 32 x 2
     // otherwise (a B200 takes about 1 us to start 1000 CTAs, so FP32's short
-    // steps want few; FP64's 156 registers leave 32 x 4 a coarser fit: 64 x 256
-    // 2.18 us against 2.16), except for a handful of CTAs, where fewer share more
-    // of the instruction stream and the L2 (16 x 40: 1.83 against 2.04; 32 x 64, 16
-    // CTAs: 2.03 against 2.06; level from 24 x 96 on).
+    // steps want few; FP64's 154 registers leave 32 x 4 a coarser fit: 64 x 256
+    // 2.22 us per step in 32 x 2 and 2.25 in 32 x 4, 256 x 1024 12.9 and 13.1), except
+    // for a dozen CTAs at most, where fewer share more of the instruction stream and
+    // the L2 (16 x 40: 1.84 in 32 x 4 against 2.06, 2.02 against 2.06 on another box;
+    // 32 x 48, 12 CTAs: 2.02 against 2.05; 32 x 64, 16: level, 2.15 against 2.09 on
+    // another box; 24 x 96: 2.07 against 2.06).
     static constexpr int BYF = std::is_same<St, float>::value ? 4 : BY;
-    static constexpr int F64_FEW_CTAS = 16;
+    static constexpr int F64_FEW_CTAS = 12;
     dim3 blk{BX, BYF}, grd{};
     // the node-pair kernel: 32 x BYX threads cover 64 columns x BYX rows
     static constexpr int BYX = X_ROWS;
