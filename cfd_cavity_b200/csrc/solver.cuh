@@ -20,9 +20,13 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <array>
+#include <cerrno>
+#include <cstdint>
 #include <type_traits>
 #include <cmath>
 #include <cstdio>
@@ -140,6 +144,24 @@ struct Solver {
     std::string err;
 };
 
+// Gives the pages of an array that is about to be written their memory in one
+// call.  Otherwise the copy from the device takes a fault at each fresh page,
+// some 3000 for the six fields of 512 x 2048, which were 11 of the 14 ms of their
+// read-back (B200 host; with this 9 to 10 ms; pages that have their memory 3 ms
+// either way).  Nothing is written, and where the kernel cannot do it (before
+// Linux 5.14, or not for this mapping) the copy faults as before.  Small arrays
+// are not worth the call.
+inline void populate_pages(void* p, size_t bytes) {
+    constexpr size_t SMALL = size_t(2) << 20;
+    constexpr int POPULATE_WRITE = 23;  // MADV_POPULATE_WRITE, which older headers lack
+    if (bytes < SMALL) return;
+    const uintptr_t page = uintptr_t(sysconf(_SC_PAGESIZE));
+    const uintptr_t a = (uintptr_t(p) + page - 1) / page * page, b = (uintptr_t(p) + bytes) / page * page;
+    const int keep = errno;
+    madvise(reinterpret_cast<void*>(a), b - a, POPULATE_WRITE);
+    errno = keep;
+}
+
 template <class St>
 struct Impl final : Solver {
     using A = typename Fmt<St>::A;
@@ -179,7 +201,8 @@ struct Impl final : Solver {
     // cavities that cannot fill the GPU (a step is then one thread's latency
     // chain; on a B200 96 x 384 f16sr 2.10 us against 2.15, 180 x 380 2.38 against
     // 2.44, 128 x 512 level), as long as every CTA runs at once: 4 of 128 threads
-    // fit on an SM, and what is left over costs a second wave (130 x 500, 750 CTAs:
+    // fit on an SM (by occupancy query: 58 registers would leave more, but its barrier
+    // numbers, not known to the compiler, reserve all 16 named barriers), and what is left over costs a second wave (130 x 500, 750 CTAs:
     // 3.40 against 2.67 with plain pairs; 4 x 2000, 1000 CTAs: 3.79 against 2.96).
     // The node limit is where plain pairs catch up in a full wave (192 x 388:
     // 2.31 against 2.28; f16g, whose g half is the longer, 128 x 590: 3.01 against 2.90)
@@ -207,9 +230,11 @@ struct Impl final : Solver {
     enum { F32_NODE = 0, F32_PAIR = 1, F32_NODE_ROUNDS = 3 };
     int f32_form = F32_NODE;
     // FP64: k_fused at 128 registers (8 CTAs of 64 threads per SM, a few
-    // words spilled) once the grid is more than the one wave that its 156
-    // registers leave room for (6 per SM): 128 x 511, 1024 CTAs, 4.50 us per
-    // step against 5.22; below that the spills cost (64 x 256: 2.67 against 2.54).
+    // words spilled) once the grid is more than the one wave that its 154
+    // registers leave room for (6 per SM): 128 x 511, 1024 CTAs, 4.23 us per
+    // step against 4.70; below that the spills cost (64 x 256: 2.60 against 2.25,
+    // 128 x 443, 888 CTAs: 3.82 against 3.59), and far above it they cost some too
+    // (256 x 1024: 13.5 against 12.9).
     static constexpr int F64_CTAS = 6, F64_PACKED_CTAS = 8;
     bool f64_packed = false;
     // dynamic subgrid model
@@ -738,7 +763,8 @@ struct Impl final : Solver {
 
     // ---- observables --------------------------------------------------------------
     // The fields, converted to dense FP64 on the device and copied straight
-    // into the caller's arrays (one synchronisation).
+    // into the caller's arrays (one synchronisation).  Large arrays are mostly
+    // pages that the caller has not touched yet, see populate_pages.
     void get_fields(double* r, double* u, double* v, double* t, double* nu_t, double* fyo) override {
         ensure_ref();
         ensure_aos();
@@ -749,6 +775,7 @@ struct Impl final : Solver {
             if (!dst[j]) continue;
             k_field_to_dense<A><<<grd, blk, 0, stream>>>(src[j], aos + j * n, G);
             check_launch();
+            populate_pages(dst[j], sizeof(double) * n);
             CK(cudaMemcpyAsync(dst[j], aos + j * n, sizeof(double) * n, cudaMemcpyDeviceToHost, stream));
         }
         CK(cudaStreamSynchronize(stream));
