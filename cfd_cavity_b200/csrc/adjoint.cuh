@@ -88,7 +88,7 @@ __global__ void k_adj_final(const St* __restrict__ X, typename Fmt<St>::A* __res
 // state), or, with every step of the sweep in the steady state (STEADY), given
 // with the launch: the table's row is a memory round trip after the step
 // counter's and the wall temperatures a third one after it, at the start of
-// every step (96 x 384 FP32 on a B200: reverse step 4.42 -> 4.20 us).
+// every step (96 x 384 FP32 on a B200: 0.22 of the reverse step's 4.2 us).
 // s = *step_dev + j in graph replays, s = j otherwise.
 template <class A>
 struct AdjScal {
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(128) k_adj_step(const St* __restrict__ X, cons
     }
     const A afy = Pin[18 * Pp + k];
     // the accumulators now: read where they are added to, they would add a
-    // memory round trip to the end of the node's chain (4.55 -> 4.42 us per step)
+    // memory round trip to the end of the node's chain (0.13 us of a step)
     const double cs0 = acc_cs[iy * nx + ix];
     const double th0 = ix == 0 ? acc_theta[iy] : 0.0;
     // 2. recompute the node's pulled inputs from X_s.

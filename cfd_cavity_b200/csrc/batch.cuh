@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(BATCH_THREADS)
 // k_fused, not of k_batch; capped at 56 (with 128-thread CTAs, 9 resident
 // per SM; a word or three spilled to L1; on a B200 +3 % binary16, +15 %
 // bfloat16 with stochastic rounding against 64 registers and 8 CTAs).  FP64's
-// node needs 156 and spills at 56: 128 there (64 cavities: 370 -> 145 us).
+// node needs 154 and spills at 56: 128 there (64 cavities: 370 us at 56, 142 at 128).
 template <class St, bool WRITE_NUT>
 __global__ void __maxnreg__((std::is_same<St, double>::value ? 128 : 56))
     k_batch_np(const BatchWork<St>* __restrict__ work, const StepScalars<typename Fmt<St>::A>* __restrict__ table,

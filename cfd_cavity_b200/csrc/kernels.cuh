@@ -129,9 +129,9 @@ __device__ __forceinline__ void store_planes(St* __restrict__ dst, const Geom& G
 // predecessor grid has completed and its writes are visible; a no-op without
 // the attribute).  The kernels leave the trigger to their exit: triggering
 // right after the wait brings the successor's CTAs onto the SMs while the
-// current step runs, where they only hold slots (B200, 128 x 512 f16sr 2.35 us
-// per step with the early trigger, 2.24 without; FP32 2.38 and 2.27; the
-// adjoint's reverse step 5.05 and 4.55; the octree's coarse step 66 and 63).
+// current step runs, where they only hold slots (B200, us per step with the early
+// trigger / without: 128 x 512 f16sr 2.34 / 2.26, FP32 2.46 / 2.20; the adjoint's
+// reverse step 4.80 / 4.22; the octree's coarse step, FP64 64 x 256, 22.2 / 20.5).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Barrier of one f warp and one g warp (or the halves of a CTA).
 __device__ __forceinline__ void named_bar_sync(int id, int threads) {

@@ -342,12 +342,10 @@ struct StepScalars {
 // significand (tests/test_const_div_cpu.py).  Below that range (|x| < 2^-968,
 // 2^-102 in binary32) the last bit may differ; the quotients are only added to
 // 1 or to a population, which absorb such a term.  The reference's expressions
-// divide about thirty times per node by these; a general division is some
-// twenty dependent operations and a branch, which cuts a node's code into
-// blocks that cannot overlap: with general divisions FP64 128 x 511 took 15.5 us
-// per step on a B200, with these 5.6 (16 x 40: 9.2 and 2.9; the block-refined
-// 64 x 256 in two levels 61 and 27 us per coarse step; 256 x 1024 in three,
-// FP32 / binary16, 91 and 75).
+// divide about thirty times per node by these.  B200, us per step of FP64 with
+// divisions / with these: 16 x 40 8.1 / 2.0, 64 x 256 8.4 / 2.2, 128 x 511 12.7 / 4.2,
+// the dynamic model on 64 x 256 18.1 / 7.5; per coarse step of the block-refined 64 x
+// 256 in two levels 53.7 / 20.0, 256 x 1024 in three 253 / 115.
 // ---------------------------------------------------------------------------
 template <class A>
 struct CsInv;  // 1/cs^2 = I2H + I2L, 1/cs^4 = I4H + I4L
@@ -398,11 +396,10 @@ CAV_OVER(over_2cs4, 0.5, I4H, I4L, A(2.0) * A(CS2) * A(CS2))
 // the approximation itself and the quotient a y, which are the division's
 // (an infinite turbulent Prandtl number: nu_t / Pr_t = 0).  Checked against the
 // division on 2^28 operand pairs (tests/test_gpu_quotient.py) and, bit for bit, on
-// those operands (tests/test_gpu_quotient_edges.py).  Code does not move across a
-// division's branch.  B200, us per step with divisions / with these: FP64 16 x 40
-// 2.36 / 2.03, 64 x 256 2.54 / 2.16, 128 x 511 4.52 / 4.30, the dynamic model on
-// 64 x 256 8.52 / 8.02; the block-refined 64 x 256 in three levels 40.3 / 37.2 per
-// coarse step (the same builds without the special operands: within 1 %).
+// those operands (tests/test_gpu_quotient_edges.py).  B200, us per step with
+// divisions / with these: FP64 16 x 40 2.31 / 2.03, 64 x 256 2.50 / 2.25, 128 x 511
+// 4.49 / 4.25, the dynamic model on 128 x 512 13.5 / 12.5; the block-refined 64 x 256 in
+// three levels 40.1 / 36.7 per coarse step.
 // ---------------------------------------------------------------------------
 // neither zero nor subnormal, infinite or NaN (an integer test: the FP64 pipe is
 // what the step waits for)
@@ -436,9 +433,9 @@ __device__ __forceinline__ double quot_rn(double a, double b, double y) {
 // first, and its root 2^100 times smaller (exactly; the remainder must not leave
 // the normal numbers); zero and infinite x come back as they are, a negative one
 // as NaN.
-// For the dynamic model's dozen independent roots (64 x 256: 8.02 -> 7.52 us per
-// step); the step itself has one, at the end of a chain, where sqrt() is the
-// shorter (2.05 us against 2.26 on 16 x 40).
+// For the dynamic model's dozen independent roots (us per step with sqrt() / with
+// this: 64 x 256 7.99 / 7.50, 128 x 512 12.9 / 12.5); the step itself has one, at the
+// end of a chain, where sqrt() is the shorter (16 x 40 2.03 us against 2.25).
 __device__ __forceinline__ double sqrt_nr(double x) {
     const int hi = __double2hiint(x);
     const double xs = __dmul_rn(x, (hi & 0x7fffffff) < 63 << 20 ? 0x1p200 : 1.0);

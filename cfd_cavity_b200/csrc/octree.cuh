@@ -93,9 +93,9 @@ struct LvlIO {
 // A level step's collision constants: with the launch once the viscosity ramp has
 // converged (STEADY; the table's row is a load after the step counter's), else
 // from the table.  The step index is only loaded where the rounding needs it.
-// B200, us per coarse step from the table / with the launch: 256 x 1024 FP32 63.1 /
-// 61.2, FP32 / binary16 58.8 / 57.4.  (k_oct_f2c keeps the table: with the
-// constants in the launch 64 x 256 FP32 took 27.8 us instead of 26.1.)
+// B200, us per coarse step from the table / with the launch: 256 x 1024 FP64 124.6 /
+// 115.1, FP32 59.6 / 58.8, FP32 / binary16 58.7 / 57.9.  (k_oct_f2c keeps the table:
+// with the constants in the launch the 64 x 256 FP32 coarse step was 6 % longer.)
 template <class A>
 struct LvlCoef {
     const OctScal<A>* tab;
@@ -523,8 +523,9 @@ __device__ __forceinline__ void split_k(int k, int nx, float inv_nx, int& x, int
 // MASK: REF and the moments are written only where L.keep is set.  L0's are read
 // by coarse_to_fine (two columns and rows along each block's edge) and by the
 // host, so every coarse step of a call but its last writes them there alone
-// (B200, 256 x 1024: 22 of 41 stores of most nodes; FP32 / binary16 57.4 -> 54.4 us per
-// coarse step, FP64 121 -> 116).  A template, and for L0 alone: the test costs the other
+// (22 of 41 stores of most nodes; B200, 256 x 1024, us per coarse step with all of
+// them / with these: FP32 62.5 / 58.8, FP32 / binary16 61.8 / 57.9, FP64 121.5 / 115.1).
+// A template, and for L0 alone: the test costs the other
 // steps more than the stores it spares (their masked nodes lie in every warp).
 template <class St, bool COARSE, bool STEADY, bool MASK>
 __global__ void __launch_bounds__(OT) k_oct_step(LvlPair<St> P, LvlCoef<typename Fmt<St>::A> lc,

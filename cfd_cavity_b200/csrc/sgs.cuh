@@ -359,8 +359,8 @@ __global__ void __launch_bounds__(128) k_sgs_b(SgsGrids<St> S, Geom G, SgsParams
 }
 
 // a^alpha b^(1 - alpha) of the mixed forms.  HALF: alpha = 1/2, as one square
-// root: eight pow were most of a node's work (64 x 256 on a B200: the part took 9.5 us of a
-// 34 us step; with this, the unrolled windows and two kernels fewer a step took 8.7).
+// root (B200, us per step with eight pow / with four roots: 64 x 256 11.5 / 7.5, 128 x
+// 512 17.7 / 12.5).
 template <bool HALF>
 __device__ __forceinline__ double sgs_mix(double a, double b, double ae) {
     if constexpr (HALF)

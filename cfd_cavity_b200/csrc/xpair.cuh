@@ -446,9 +446,10 @@ __global__ void __launch_bounds__(64 * XS_ROWS) k_fused_xs(const St* __restrict_
 }
 
 // The single-cavity step on node pairs: a CTA covers 64 columns x X_ROWS rows.
-// X_CTAS resident CTAs leave 104 registers (18 warps per SM).  B200, 512 x 2048
-// f16sr: 14.9 us per step; at 10 CTAs and 96 registers 15.2, at 98 registers
-// without the bound 16.3, at 11 and 12 CTAs 15.5.
+// The bound of X_CTAS CTAs per SM lets the compiler schedule for up to 112 registers;
+// it uses 94 or 95, and 10 CTAs (20 warps) are resident.  B200, 512 x 2048 f16sr, us
+// per step by the bound: 9: 14.9, 10: 15.2 (96 registers), 11 and 12: 15.5, none: 16.3
+// (98 registers).
 constexpr int X_ROWS = 2, X_CTAS = 9;
 template <class St, bool WRITE_NUT, bool ACC_NU, bool NO_COLLIDE>
 __global__ void __launch_bounds__(32 * X_ROWS, X_CTAS) k_fused_x(const St* __restrict__ src, St* __restrict__ dst,
