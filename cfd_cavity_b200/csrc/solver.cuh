@@ -188,9 +188,9 @@ struct Impl final : Solver {
     // steps want few; FP64's 154 registers leave 32 x 4 a coarser fit: 64 x 256
     // 2.22 us per step in 32 x 2 and 2.25 in 32 x 4, 256 x 1024 12.9 and 13.1), except
     // for a dozen CTAs at most, where fewer share more of the instruction stream and
-    // the L2 (16 x 40: 1.84 in 32 x 4 against 2.06, 2.02 against 2.06 on another box;
+    // the L2 (16 x 40: 1.84 in 32 x 4 against 2.06, 2.02 against 2.06 on another B200;
     // 32 x 48, 12 CTAs: 2.02 against 2.05; 32 x 64, 16: level, 2.15 against 2.09 on
-    // another box; 24 x 96: 2.07 against 2.06).
+    // another B200; 24 x 96: 2.07 against 2.06).
     static constexpr int BYF = std::is_same<St, float>::value ? 4 : BY;
     static constexpr int F64_FEW_CTAS = 12;
     dim3 blk{BX, BYF}, grd{};
