@@ -202,8 +202,9 @@ struct Impl final : Solver {
     // chain; on a B200 96 x 384 f16sr 2.10 us against 2.15, 180 x 380 2.38 against
     // 2.44, 128 x 512 level), as long as every CTA runs at once: 4 of 128 threads
     // fit on an SM (by occupancy query: 58 registers would leave more, but its barrier
-    // numbers, not known to the compiler, reserve all 16 named barriers), and what is left over costs a second wave (130 x 500, 750 CTAs:
-    // 3.40 against 2.67 with plain pairs; 4 x 2000, 1000 CTAs: 3.79 against 2.96).
+    // numbers, not known to the compiler, reserve all 16 named barriers), and what is
+    // left over costs a second wave (130 x 500, 750 CTAs: 3.40 against 2.67 with plain
+    // pairs; 4 x 2000, 1000 CTAs: 3.79 against 2.96).
     // The node limit is where plain pairs catch up in a full wave (192 x 388:
     // 2.31 against 2.28; f16g, whose g half is the longer, 128 x 590: 3.01 against 2.90)
     static constexpr int SPLIT_CTAS = 4;
